@@ -246,11 +246,10 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_adj_c2r(Geo g, const 
     double2 *buf = sm, *tws = sm + L::BUF;
     load_tw<N>(tws, g);
     const int i = blockIdx.x / L::C, rank = blockIdx.x % L::C, item = blockIdx.y, nx = g.nx;
-    const TwT tw{tws, N};
     for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
         const int kz = e / L::PZ, jl = e - kz * L::PZ;
         if (jl == L::MC && rank != 0) continue;
-        const int j = cl_col<N>(jl, rank), ge = kz * my2 + j;
+        const int j = cl_col<L>(jl, rank), ge = kz * my2 + j;
         const double s = 1.0 / (cky(j, N) * g.nrm);
         double2 v;
         if (mode == 0) {
@@ -270,16 +269,16 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_adj_c2r(Geo g, const 
         buf[e] = make_double2(v.x * s, v.y * s);
     }
     __syncthreads();
-    cl_c2r<N>(buf, tw, rank);
-    if (threadIdx.x == 0) { bulk_store(dst + ((size_t)item * nx + i) * RSP + (size_t)rank * L::RL, buf, L::RBYTES); bulk_wait_read(); }
+    cl_c2r<L>(buf, tws, rank);
+    if (threadIdx.x == 0) { bulk_store(dst + ((size_t)item * nx + i) * RSP + (size_t)rank * L::ROWS, buf, L::RBYTES); bulk_wait_read(); }
 }
 
 // k_adj_r2c: transposes of the step's c2r transforms, c2r^T(r) = c_ky (my mz) r2c(r),
 // over nplanes consecutive real planes (grid.x = nplanes * C).
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_adj_r2c(Geo g, const double *__restrict__ src, double2 *__restrict__ dst,
+__global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) k_adj_r2c(Geo g, const double *__restrict__ src, double2 *__restrict__ dst,
                                                         AdjScal *as) {
-    using L = PL<N>;
+    using L = RL<N>;
     extern __shared__ double2 sm[];
     constexpr int my2 = N / 2 + 1, PS = my2 * N, RSP = RP<N>::RSP;
     double2 *buf = sm, *tws = sm + L::BUF;
@@ -290,22 +289,19 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_adj_r2c(Geo g, const 
     const uint32_t phase = 0;
     const size_t pl = blockIdx.x / L::C;
     const int rank = blockIdx.x % L::C;
-    const TwT tw{tws, N};
     if (threadIdx.x == 0) {
         fence_async_smem();
-        bulk_load(buf, src + pl * RSP + (size_t)rank * L::RL, L::RBYTES, &mb);
+        bulk_load(buf, src + pl * RSP + (size_t)rank * L::ROWS, L::RBYTES, &mb);
     }
     if (!mbar_wait(&mb, phase)) atomicCAS(&as->status, 0, PIBM_ERR_TIMEOUT);
     __syncthreads();
-    cl_r2c<N>(buf, tw, rank);
-    for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
-        const int kz = e / L::PZ, jl = e - kz * L::PZ;
-        if (jl == L::MC && rank != 0) continue;
-        const int j = cl_col<N>(jl, rank);
-        const double2 X = cl_unpack<N>(buf, kz, jl, rank);
+    cl_r2c_out<L>(buf, tws, rank, [&](int kz, int step, int jl, const double2 *X, auto n) {
+        const int j = cl_col<L>(jl, rank);
         const double c = cky(j, N);
-        dst[pl * PS + kz * my2 + j] = make_double2(X.x * c, X.y * c);
-    }
+        double2 *d = dst + pl * PS + kz * my2 + j;
+#pragma unroll
+        for (int k = 0; k < decltype(n)::value; ++k) d[k * step * my2] = make_double2(X[k].x * c, X[k].y * c);
+    });
 }
 
 // Sum over the nodes of component blockIdx.y of a real field (row padding
@@ -717,7 +713,7 @@ static void enqueue_adjoint_step_t(const Geo &g, const DevBufs &b, const AdjBufs
     k_adj_begin<<<1, 32, 0, s>>>(b.sc, a.as);
     k_adj_lines<N, LT><<<(g.PS + LT - 1) / LT, LT * 32, adj_lines_smem<N>(), s>>>(g, a.lu, a.lp, a.lnl, a.lu2, a.lp2, a.lnl_new,
                                                                                  a.lonl, a.lff, b.sc, a.as);
-    launch_planes<N>(k_adj_c2r<N>, g.nx, 3, s, g, (const double2 *)a.lff, a.lfr, 0);
+    launch_planes<PL<N>>(k_adj_c2r<N>, g.nx, 3, s, g, (const double2 *)a.lff, a.lfr, 0);
     k_adj_sum<N><<<dim3(nsum, 3), 256, 0, s>>>(g, a.lfr, lfrmean, -1.0);
     cudaMemsetAsync(a.lubcp, 0, 10 * CR * sizeof(double), s);   // lubcp, lomega, lpbcp, lpgr
     cudaMemsetAsync(a.lQ, 0, 3 * CR * sizeof(double), s);
@@ -725,12 +721,12 @@ static void enqueue_adjoint_step_t(const Geo &g, const DevBufs &b, const AdjBufs
         k_adj_rev<N><<<(g.npts + 255) / 256, 256, 0, s>>>(g, b.ubcp, b.pgr, b.Q, b.rec, a.lfr, b.sc, a.as, a.lubcp, a.lQ, a.lpgr, a.gxc);
     if (wJ != 0.0)   // RK3: only the step's last stage carries the objective
         k_adj_drag<N><<<(g.nbody * g.nbnd + 255) / 256, 256, 0, s>>>(g, b.pbcp, b.omega, a.lpbcp, a.lomega, a.gxc, e[0], e[1], e[2], wJ);
-    launch_planes<N>(k_adj_r2c<N>, 3 * g.nx, 1, s, g, (const double *)a.lQ, a.T, a.as);
+    launch_planes<RL<N>>(k_adj_r2c<N>, 3 * g.nx, 1, s, g, (const double *)a.lQ, a.T, a.as);
     k_adj_q<<<(unsigned)((3 * SC + 255) / 256), 256, 0, s>>>(g, a.T, a.lnl_new, a.lonl, a.lu2);
-    launch_planes<N>(k_adj_c2r<N>, g.nx, 8, s, g, (const double2 *)a.lnl_new, a.W8, 1);
+    launch_planes<PL<N>>(k_adj_c2r<N>, g.nx, 8, s, g, (const double2 *)a.lnl_new, a.W8, 1);
     k_adj_flux<N><<<(unsigned)((RP<N>::RSP * (g.nx / kAdjFluxSeg) + 255) / 256), 256, 0, s>>>(g, b.ubcp, a.W8, a.lubcp);
     k_adj_sum<N><<<dim3(nsum, 3), 256, 0, s>>>(g, a.lubcp, lumean, 1.0);
-    launch_planes<N>(k_adj_r2c<N>, 10 * g.nx, 1, s, g, (const double *)a.lubcp, a.T, a.as);
+    launch_planes<RL<N>>(k_adj_r2c<N>, 10 * g.nx, 1, s, g, (const double *)a.lubcp, a.T, a.as);
     k_adj_assemble<<<(unsigned)((SC + 255) / 256), 256, 0, s>>>(g, a.T, a.lu2, a.lp2);
 }
 
@@ -751,10 +747,10 @@ void enqueue_adjoint_jacc(const Scal *sc, AdjScal *as, const double e[3], cudaSt
 
 template <int N>
 static cudaError_t set_adj_attrs() {
-    const int maxs = (int)plane_smem<N>();
+    const int maxs = (int)PL<N>::SMEM;
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(k_adj_c2r<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_adj_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_adj_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
     constexpr int LT = N >= 256 ? 4 : 8;
     return cudaFuncSetAttribute(k_adj_lines<N, LT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_lines_smem<N>());
 }

@@ -65,8 +65,7 @@ __device__ __forceinline__ void b_a0(const Geo &g, const double2 *__restrict__ u
     grid_dep_wait();   // the twiddles above are set-up data; the fields come from earlier kernels
     const int i = blockIdx.x / L::C, rank = blockIdx.x % L::C, nx = g.nx;
     const int im = (i - 1 + nx) % nx, ip = (i + 1) % nx;
-    const size_t roff = (size_t)rank * L::RL;
-    const TwT tw{tws, N};
+    const size_t roff = (size_t)rank * L::ROWS;
     const double tdx = 2.0 * g.dx, rtdx = 1.0 / tdx;   // divisor and reciprocal for qdiv
     const double2 *U0 = u + (size_t)i * PS, *U1 = u + ((size_t)nx + i) * PS, *U2 = u + ((size_t)2 * nx + i) * PS;
     const double2 *Pp = p + (size_t)i * PS;
@@ -74,15 +73,9 @@ __device__ __forceinline__ void b_a0(const Geo &g, const double2 *__restrict__ u
     {
         const int t = blockIdx.y;
         if (t < 4) {
-            // a plain copy of u_t or p: the CTA's MC columns of every kz row as N
-            // bulk copies into the padded rows, all in flight at once; rank 0's
-            // Nyquist column (slot MC) with plain loads beside them
-            const double2 *src = t == 0 ? U0 : t == 1 ? U1 : t == 2 ? U2 : Pp;
+            // a plain copy of u_t or p
             uint32_t phase = 0;
-            if (threadIdx.x < 32)
-                bulk_load_rows(buf, L::PZ * 16, src + rank * L::MC, (size_t)my2 * 16, L::MC * 16, N, &mb);
-            if (rank == 0)
-                for (int kz = threadIdx.x; kz < N; kz += L::T) buf[kz * L::PZ + L::MC] = src[kz * my2 + L::M];
+            load_plane<L>(buf, t == 0 ? U0 : t == 1 ? U1 : t == 2 ? U2 : Pp, rank, &mb);
             load_wait(&mb, phase, sc);
         } else {
             // omega and grad p: spectral differences formed from plain loads
@@ -90,7 +83,7 @@ __device__ __forceinline__ void b_a0(const Geo &g, const double2 *__restrict__ u
             for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
                 const int kz = e / L::PZ, jl = e - kz * L::PZ;
                 if (jl == L::MC && rank != 0) continue;
-                const int j = cl_col<N>(jl, rank), ge = kz * my2 + j;
+                const int j = cl_col<L>(jl, rank), ge = kz * my2 + j;
                 const double ky = g.ky[j], kzv = g.kz[kz];
                 double2 f;
                 if (t == 4) {   // wy*u3 - wz*u2
@@ -115,14 +108,14 @@ __device__ __forceinline__ void b_a0(const Geo &g, const double2 *__restrict__ u
             }
         }
         __syncthreads();
-        cl_c2r<N>(buf, tw, rank);
+        cl_c2r<L>(buf, tws, rank);
         if (t < 3) {
             // u + umean; fluid, solid and total sums and max |u| of this CTA's rows
             const double um = sc->umean[t];
             double *b = (double *)buf;
             const uint8_t *fl = g.fluid + (size_t)i * RSP + roff;
             double sf = 0.0, ss = 0.0, sa = 0.0, mx = kSmallD;
-            for (int e = threadIdx.x; e < L::RL; e += L::T) {
+            for (int e = threadIdx.x; e < L::ROWS; e += L::T) {
                 if (e % (N + 2) >= N) continue;
                 const double v = b[e] + um;
                 b[e] = v;
@@ -382,7 +375,7 @@ __device__ __forceinline__ void b_nl(const Geo &g, const double *__restrict__ ub
                                                    const double2 *__restrict__ u,
                                                    const double2 *__restrict__ onl, double2 *__restrict__ nl_new,
                                                    double *__restrict__ Q, Scal *__restrict__ sc) {
-    using L = PL<N>;
+    using L = NL<N>;
     extern __shared__ double2 sm[];
     constexpr int my2 = N / 2 + 1, PS = my2 * N, RS = RP<N>::RSP;
     double2 *buf = sm, *tws = sm + L::BUF;
@@ -394,8 +387,7 @@ __device__ __forceinline__ void b_nl(const Geo &g, const double *__restrict__ ub
     uint32_t phase = 0;
     const int i = blockIdx.x / L::C, rank = blockIdx.x % L::C, nx = g.nx;
     const int im = (i - 1 + nx) % nx, ip = (i + 1) % nx;
-    const size_t roff = (size_t)rank * L::RL;
-    const TwT tw{tws, N};
+    const size_t roff = (size_t)rank * L::ROWS;
     // real component n of this CTA's rows
     auto Uc = [&](int n) { return ubcp + ((size_t)n * nx + i) * RS + roff; };
     const double c12 = g.c1 + g.c2;
@@ -417,7 +409,7 @@ __device__ __forceinline__ void b_nl(const Geo &g, const double *__restrict__ ub
                 double2 *b2 = buf;
                 const double2 *B2 = (const double2 *)Uc(nb);
 #pragma unroll 8
-                for (int e = threadIdx.x; e < L::RL / 2; e += L::T) {
+                for (int e = threadIdx.x; e < L::ROWS / 2; e += L::T) {
                     const double2 x = b2[e], y = B2[e];
                     b2[e] = make_double2(x.x * y.x, x.y * y.y);
                 }
@@ -429,19 +421,27 @@ __device__ __forceinline__ void b_nl(const Geo &g, const double *__restrict__ ub
                 }
                 load_wait(&mb, phase, sc);
             }
-            cl_r2c<N>(buf, tw, rank);
             if (q < 2) {
-#pragma unroll 4
-                for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
-                    const int kz = e / L::PZ, jl = e - kz * L::PZ;
-                    if (jl == L::MC && rank != 0) continue;
-                    const int ge = kz * my2 + cl_col<N>(jl, rank);
-                    const double2 Xr = cl_unpack<N>(buf, kz, jl, rank);
-                    const double2 X = r2c_norm<N>(Xr, g.nrm);
-                    if (q == 0) { const double ky = g.ky[cl_col<N>(jl, rank)]; dst[ge] = make_double2(-ky * X.y, ky * X.x); }
-                    else { const double kzv = g.kz[kz]; dst[ge] = cadd(dst[ge], make_double2(-kzv * X.y, kzv * X.x)); }
-                }
+                cl_r2c_out<L>(buf, tws, rank, [&](int kz, int step, int jl, const double2 *X, auto n) {
+                    const int j = cl_col<L>(jl, rank), ge = kz * my2 + j;
+                    if (q == 0) {
+                        const double ky = g.ky[j];
+#pragma unroll
+                        for (int k = 0; k < decltype(n)::value; ++k) {
+                            const double2 x = r2c_norm<N>(X[k], g.nrm);
+                            dst[ge + k * step * my2] = make_double2(-ky * x.y, ky * x.x);
+                        }
+                    } else {
+                        update_piece(dst, ge, step * my2, n, [&](int k, double2 d) {
+                            const double2 x = r2c_norm<N>(X[k], g.nrm);
+                            const double kzv = g.kz[kz + k * step];
+                            return cadd(d, make_double2(-kzv * x.y, kzv * x.x));
+                        });
+                    }
+                });
                 __syncthreads();
+            } else {
+                cl_r2c<L>(buf, tws, rank);
             }
         }
         // nl = -(...) (nl.F90:146-152); Q = -c3 nl - c4 onl - c12 diffn (calc_visc spectrum)
@@ -449,8 +449,8 @@ __device__ __forceinline__ void b_nl(const Geo &g, const double *__restrict__ ub
         const double2 *uc = u + (size_t)c * nx * PS;
         // the nl value of element (kz, jl) and the transform input of Q there
         auto nl_q = [&](int kz, int jl) -> double2 {
-            const int ge = kz * my2 + cl_col<N>(jl, rank);
-            const double2 X = r2c_norm<N>(cl_unpack<N>(buf, kz, jl, rank), g.nrm);
+            const int ge = kz * my2 + cl_col<L>(jl, rank);
+            const double2 X = r2c_norm<N>(cl_unpack<L>(buf, kz, jl, rank), g.nrm);
             const double2 s = cadd(dst[ge], X);
             const double2 v = make_double2(-s.x, -s.y);
             dst[ge] = v;
@@ -486,12 +486,12 @@ __device__ __forceinline__ void b_nl(const Geo &g, const double *__restrict__ ub
             }
         }
         __syncthreads();
-        cl_c2r<N>(buf, tw, rank);
+        cl_c2r<L>(buf, tws, rank);
         if (threadIdx.x == 0) { bulk_store(Q + ((size_t)c * nx + i) * RS + roff, buf, L::RBYTES); bulk_wait_read(); }
     }
 }
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_nl(Geo g, const double *__restrict__ ubcp, const double *__restrict__ Dx,
+__global__ void __launch_bounds__(NL<N>::T, NL<N>::MINB) k_nl(Geo g, const double *__restrict__ ubcp, const double *__restrict__ Dx,
                                                    const double2 *__restrict__ u,
                                                    const double2 *__restrict__ onl, double2 *__restrict__ nl_new,
                                                    double *__restrict__ Q, Scal *__restrict__ sc) { b_nl<N>(g, ubcp, Dx, u, onl, nl_new, Q, sc); }
@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(256) k_spread(Geo g, const double *__restrict_
 template <int N>
 __device__ __forceinline__ void b_ff(const Geo &g, const double *__restrict__ fr, double2 *__restrict__ ff,
                                                    Scal *__restrict__ sc) {
-    using L = PL<N>;
+    using L = RL<N>;
     extern __shared__ double2 sm[];
     constexpr int my2 = N / 2 + 1, PS = my2 * N, RSP = RP<N>::RSP;
     double2 *buf = sm, *tws = sm + L::BUF;
@@ -807,8 +807,7 @@ __device__ __forceinline__ void b_ff(const Geo &g, const double *__restrict__ fr
     grid_dep_wait();   // the twiddles above are set-up data; the fields come from earlier kernels
     uint32_t phase = 0;
     const int i = blockIdx.x / L::C, rank = blockIdx.x % L::C, nx = g.nx;
-    const size_t roff = (size_t)rank * L::RL;
-    const TwT tw{tws, N};
+    const size_t roff = (size_t)rank * L::ROWS;
     {
         const int n = blockIdx.y;
         if (threadIdx.x == 0) {
@@ -818,21 +817,18 @@ __device__ __forceinline__ void b_ff(const Geo &g, const double *__restrict__ fr
         load_wait(&mb, phase, sc);
         const double fmn = sc->frmean[n];
         double *b = (double *)buf;
-        for (int e = threadIdx.x; e < L::RL; e += L::T) b[e] = b[e] - fmn;
+        for (int e = threadIdx.x; e < L::ROWS; e += L::T) b[e] = b[e] - fmn;
         __syncthreads();
-        cl_r2c<N>(buf, tw, rank);
         double2 *dst = ff + ((size_t)n * nx + i) * PS;
-#pragma unroll 4
-        for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
-            const int kz = e / L::PZ, jl = e - kz * L::PZ;
-            if (jl == L::MC && rank != 0) continue;
-            const double2 X = cl_unpack<N>(buf, kz, jl, rank);
-            dst[kz * my2 + cl_col<N>(jl, rank)] = r2c_norm<N>(X, g.nrm);
-        }
+        cl_r2c_out<L>(buf, tws, rank, [&](int kz, int step, int jl, const double2 *X, auto n) {
+            double2 *d = dst + kz * my2 + cl_col<L>(jl, rank);
+#pragma unroll
+            for (int k = 0; k < decltype(n)::value; ++k) d[k * step * my2] = r2c_norm<N>(X[k], g.nrm);
+        });
     }
 }
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_ff(Geo g, const double *__restrict__ fr, double2 *__restrict__ ff,
+__global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) k_ff(Geo g, const double *__restrict__ fr, double2 *__restrict__ ff,
                                                    Scal *__restrict__ sc) { b_ff<N>(g, fr, ff, sc); }
 
 // ============================================================================
@@ -1100,16 +1096,16 @@ static int sm_count() {
 // launch_planes with programmatic dependent launch: the blocks may start
 // (and run the prologue before their grid_dep_wait) while the previous kernel
 // of the stream drains.
-template <int N, typename... KArgs, typename... Args>
+template <class L, typename... KArgs, typename... Args>
 inline void launch_planes_pdl(void (*k)(KArgs...), int nplanes, int items, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(nplanes * PL<N>::C), (unsigned)items, 1);
-    cfg.blockDim = dim3(PL<N>::T, 1, 1);
-    cfg.dynamicSmemBytes = plane_smem<N>();
+    cfg.gridDim = dim3((unsigned)(nplanes * L::C), (unsigned)items, 1);
+    cfg.blockDim = dim3(L::T, 1, 1);
+    cfg.dynamicSmemBytes = L::SMEM;
     cfg.stream = s;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = PL<N>::C;
+    at[0].val.clusterDim.x = L::C;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1203,6 +1199,17 @@ __global__ void k_d2f(const double2 *__restrict__ d, double2 *__restrict__ f, in
 
 // Standalone batched plane transforms (pibm_ff2rc / pibm_ff2cr) on natural
 // host layouts: real a[z*my + y], complex b[kz*my2 + ky].
+// f(r, m): row r of the CTA's row phase and real pair m (values y = 2m, 2m+1).
+// A warp takes 8 rows x 4 consecutive pairs: 8 rows at one pair lie in
+// distinct banks (odd pitch), and a row's 4 pairs are 64 contiguous bytes of
+// the natural plane.
+template <class L, class F> __device__ __forceinline__ void for_real_pairs(F f) {
+    static_assert(L::NR % 8 == 0 && L::M % 4 == 0, "8 x 4 blocks");
+    for (int e = threadIdx.x; e < L::NR * L::M; e += L::T) {
+        const int w = e >> 5;
+        f((w % (L::NR / 8)) * 8 + (e & 7), (w / (L::NR / 8)) * 4 + ((e >> 3) & 3));
+    }
+}
 template <int N>
 __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_ff2cr(Geo g, const double2 *__restrict__ a, double *__restrict__ b) {
     using L = PL<N>;
@@ -1210,47 +1217,42 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_ff2cr(Geo g, const do
     constexpr int my2 = N / 2 + 1, PS = my2 * N, RS = N * N;
     double2 *buf = sm, *tws = sm + L::BUF;
     load_tw<N>(tws, g);
-    const TwT tw{tws, N};
     const size_t q = blockIdx.x / L::C;
     const int rank = blockIdx.x % L::C;
     for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
         const int kz = e / L::PZ, jl = e - kz * L::PZ;
         if (jl == L::MC && rank != 0) continue;
-        buf[e] = a[q * PS + kz * my2 + cl_col<N>(jl, rank)];
+        buf[e] = a[q * PS + kz * my2 + cl_col<L>(jl, rank)];
     }
     __syncthreads();
-    cl_c2r<N>(buf, tw, rank);
-    const double *rb = (const double *)buf;
-    for (int e = threadIdx.x; e < L::NR * N; e += L::T) {
-        const int r = e / N, y = e - r * N;
-        const int z = zinv<N>(rank * L::NR + r);
-        b[q * RS + (size_t)z * N + y] = rb[r * (N + 2) + 2 * yslot<N>(y >> 1) + (y & 1)];
-    }
+    cl_c2r<L>(buf, tws, rank);
+    double *dst = b + q * RS;
+    const bool wide = ((uintptr_t)b & 15) == 0;   // the caller's buffer need only be aligned to its doubles
+    for_real_pairs<L>([&](int r, int m) {
+        const double2 v = buf[r * L::P + yslot<N>(m)];
+        double *d = dst + (size_t)zinv<N>(rank * L::NR + r) * N + 2 * m;
+        if (wide) *(double2 *)d = v;
+        else { d[0] = v.x; d[1] = v.y; }
+    });
 }
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_ff2rc(Geo g, const double *__restrict__ a, double2 *__restrict__ b) {
-    using L = PL<N>;
+__global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) k_ff2rc(Geo g, const double *__restrict__ a, double2 *__restrict__ b) {
+    using L = RL<N>;
     extern __shared__ double2 sm[];
     constexpr int my2 = N / 2 + 1, PS = my2 * N, RS = N * N;
     double2 *buf = sm, *tws = sm + L::BUF;
     load_tw<N>(tws, g);
-    const TwT tw{tws, N};
     const size_t q = blockIdx.x / L::C;
     const int rank = blockIdx.x % L::C;
-    double *rb = (double *)buf;
-    for (int e = threadIdx.x; e < L::NR * N; e += L::T) {
-        const int r = e / N, y = e - r * N;
-        const int z = zinv<N>(rank * L::NR + r);
-        rb[r * (N + 2) + 2 * yslot<N>(y >> 1) + (y & 1)] = a[q * RS + (size_t)z * N + y];
-    }
+    for_real_pairs<L>([&](int r, int m) {
+        buf[r * L::P + yslot<N>(m)] = *(const double2 *)(a + q * RS + (size_t)zinv<N>(rank * L::NR + r) * N + 2 * m);
+    });
     __syncthreads();
-    cl_r2c<N>(buf, tw, rank);
-    for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
-        const int kz = e / L::PZ, jl = e - kz * L::PZ;
-        if (jl == L::MC && rank != 0) continue;
-        const double2 X = cl_unpack<N>(buf, kz, jl, rank);
-        b[q * PS + kz * my2 + cl_col<N>(jl, rank)] = r2c_norm<N>(X, g.nrm);
-    }
+    cl_r2c_out<L>(buf, tws, rank, [&](int kz, int step, int jl, const double2 *X, auto n) {
+        double2 *d = b + q * PS + kz * my2 + cl_col<L>(jl, rank);
+#pragma unroll
+        for (int k = 0; k < decltype(n)::value; ++k) d[k * step * my2] = r2c_norm<N>(X[k], g.nrm);
+    });
 }
 
 // ============================================================================
@@ -1278,7 +1280,7 @@ __global__ void __launch_bounds__(256, 4) kb_flux(const __grid_constant__ Member
     b_flux<N>(m.g, m.b.ubcp, m.b.Dx, m.b.sc);
 }
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) kb_nl(const __grid_constant__ MemberSet ms) {
+__global__ void __launch_bounds__(NL<N>::T, NL<N>::MINB) kb_nl(const __grid_constant__ MemberSet ms) {
     const Member &m = ms.m[blockIdx.z];
     b_nl<N>(m.g, m.b.ubcp, m.b.Dx, m.b.u, m.b.nl[m.cur ^ 1], m.b.nl[m.cur], m.b.Q, m.b.sc);
 }
@@ -1310,7 +1312,7 @@ __global__ void __launch_bounds__(256) kb_spread(const __grid_constant__ MemberS
     b_spread(m.g, m.b.rec, m.b.rz, m.b.fr, m.b.sc);
 }
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) kb_ff(const __grid_constant__ MemberSet ms) {
+__global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) kb_ff(const __grid_constant__ MemberSet ms) {
     const Member &m = ms.m[blockIdx.z];
     if (m.g.nbody == 0) return;
     b_ff<N>(m.g, m.b.fr, m.b.ff, m.b.sc);
@@ -1335,7 +1337,7 @@ template <int N>
 static void enqueue_batch_step_t(const MemberSet &ms, const BatchShape &bs, cudaStream_t s, cudaStream_t side,
                                  cudaEvent_t fork, cudaEvent_t join) {
     const int nz = bs.nz;
-    launch_planes_z<N>(kb_a0<N>, N, 10, nz, s, ms);
+    launch_planes_z<PL<N>>(kb_a0<N>, N, 10, nz, s, ms);
     const bool spheres = bs.max_nbody > 0;
     cudaEventRecord(fork, s);
     cudaStreamWaitEvent(side, fork, 0);
@@ -1346,7 +1348,7 @@ static void enqueue_batch_step_t(const MemberSet &ms, const BatchShape &bs, cuda
     }
     cudaEventRecord(join, side);
     kb_flux<N><<<dim3((RP<N>::RSP * (N / bs.flux_seg) + 255) / 256, 1, nz), 256, 0, s>>>(ms);
-    launch_planes_z<N>(kb_nl<N>, N, 3, nz, s, ms);
+    launch_planes_z<NL<N>>(kb_nl<N>, N, 3, nz, s, ms);
     cudaStreamWaitEvent(s, join, 0);
     if (spheres) {
         if (bs.max_nbk > 0) {
@@ -1358,7 +1360,7 @@ static void enqueue_batch_step_t(const MemberSet &ms, const BatchShape &bs, cuda
             if (bs.max_spn > 0) kb_spread<<<dim3((bs.max_spn + 255) / 256, 1, nz), 256, 0, s>>>(ms);
             cudaStreamWaitEvent(s, join, 0);
         }
-        launch_planes_z<N>(kb_ff<N>, N, 3, nz, s, ms);
+        launch_planes_z<RL<N>>(kb_ff<N>, N, 3, nz, s, ms);
     }
     const int PS = (N / 2 + 1) * N;
     if (bs.lines_lt == 4) kb_lines<N, 4><<<dim3((PS + 3) / 4, 1, nz), 4 * 32, lines_smem<N>(4), s>>>(ms);
@@ -1386,20 +1388,20 @@ int batch_kernels_per_step(const BatchShape &bs) {
 // ============================================================================
 template <int N>
 static cudaError_t set_attrs() {
-    const int maxs = (int)plane_smem<N>();
+    const int maxs = (int)PL<N>::SMEM;
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(k_a0<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_nl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_ff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_nl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NL<N>::SMEM)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_ff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_ff2cr<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_ff2rc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_ff2rc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_lines<N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lines_smem<N>(4))) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_lines<N, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lines_smem<N>(8))) != cudaSuccess) return e;
     if constexpr (N <= 128)
         if ((e = cudaFuncSetAttribute(k_lines_pipe<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, LPipe<N>::SMEM)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(kb_a0<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_nl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_ff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(kb_nl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NL<N>::SMEM)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(kb_ff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(kb_lines<N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lines_smem<N>(4))) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(kb_lines<N, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lines_smem<N>(8))) != cudaSuccess) return e;
     return cudaSuccess;
@@ -1467,7 +1469,7 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
     const bool scal_first = g.scal && !g.moving;
     mark(0);
     kb(PIBM_K_A0);
-    launch_planes_pdl<N>(k_a0<N>, g.nx, 10, s, g, (const double2 *)b.u, (const double2 *)b.p, b.ubcp, b.pbcp, b.omega, b.pgr, b.sc, b.part);
+    launch_planes_pdl<PL<N>>(k_a0<N>, g.nx, 10, s, g, (const double2 *)b.u, (const double2 *)b.p, b.ubcp, b.pbcp, b.omega, b.pgr, b.sc, b.part);
     ke(PIBM_K_A0);
     if (fork) {
         if (scal_first) k_scal_a<<<1, 256, 0, s>>>(g, b.sc, b.part);
@@ -1497,7 +1499,7 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
     else k_flux<N, 4><<<fgrid, 256, 0, s>>>(g, b.ubcp, b.Dx, b.sc);
     ke(PIBM_K_FLUX);
     kb(PIBM_K_NL);
-    launch_planes_pdl<N>(k_nl<N>, g.nx, 3, s, g, (const double *)b.ubcp, (const double *)b.Dx, (const double2 *)b.u,
+    launch_planes_pdl<NL<N>>(k_nl<N>, g.nx, 3, s, g, (const double *)b.ubcp, (const double *)b.Dx, (const double2 *)b.u,
                          (const double2 *)b.nl[old], b.nl[cur], b.Q, b.sc);
     ke(PIBM_K_NL);
     mark(2);
@@ -1548,7 +1550,7 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
         }
         mark(4);
         kb(PIBM_K_FF);
-        launch_planes_pdl<N>(k_ff<N>, g.nx, 3, s, g, (const double *)b.fr, b.ff, b.sc);
+        launch_planes_pdl<RL<N>>(k_ff<N>, g.nx, 3, s, g, (const double *)b.fr, b.ff, b.sc);
         ke(PIBM_K_FF);
     } else {
         mark(3); mark(4);
@@ -1591,7 +1593,7 @@ void enqueue_step(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cudaEvent_t
 
 template <int N>
 static void enqueue_c2r_t(const Geo &g, const double2 *a, double *b, int nplanes, cudaStream_t s) {
-    launch_planes<N>(k_ff2cr<N>, nplanes, 1, s, g, a, b);
+    launch_planes<PL<N>>(k_ff2cr<N>, nplanes, 1, s, g, a, b);
 }
 void enqueue_c2r(const Geo &g, const double2 *a, double *b, int nplanes, cudaStream_t s) {
     switch (g.my) {
@@ -1604,7 +1606,7 @@ void enqueue_c2r(const Geo &g, const double2 *a, double *b, int nplanes, cudaStr
 }
 template <int N>
 static void enqueue_r2c_t(const Geo &g, const double *a, double2 *b, int nplanes, cudaStream_t s) {
-    launch_planes<N>(k_ff2rc<N>, nplanes, 1, s, g, a, b);
+    launch_planes<RL<N>>(k_ff2rc<N>, nplanes, 1, s, g, a, b);
 }
 void enqueue_r2c(const Geo &g, const double *a, double2 *b, int nplanes, cudaStream_t s) {
     switch (g.my) {
@@ -1686,7 +1688,7 @@ static cudaError_t autotune_lines_t(Geo &g, DevBufs &b, int cur, cudaStream_t s,
                 // the forcing transform writes only the work field ff, which the
                 // step recomputes before its line kernel; runs without
                 // particles have no forcing (fr is not allocated, ff stays zero)
-                if (g.nbody > 0 && b.fr) launch_planes<N>(k_ff<N>, g.nx, 3, s, g, (const double *)b.fr, b.ff, sc);
+                if (g.nbody > 0 && b.fr) launch_planes<RL<N>>(k_ff<N>, g.nx, 3, s, g, (const double *)b.fr, b.ff, sc);
                 launch_lines<N>(gt, b, u, p, cur, sc, s);
             }
         };

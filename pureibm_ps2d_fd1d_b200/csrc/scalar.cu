@@ -44,12 +44,12 @@ __device__ __forceinline__ double2 phi_at(const Geo &g, const double2 *__restric
 // (nl_allphi.F90:96-114, 256-330; bc_scalar.F90:935-1033, serial branches)
 // ============================================================================
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_sa(Geo g, const double2 *__restrict__ phif,
+__global__ void __launch_bounds__(SL<N>::T, SL<N>::MINB) k_sa(Geo g, const double2 *__restrict__ phif,
                                                               const double *__restrict__ ubcp, double *__restrict__ phr,
                                                               double *__restrict__ phimg, double *__restrict__ sdf,
                                                               double *__restrict__ gph, const Scal *__restrict__ sc,
                                                               double *__restrict__ spart) {
-    using L = PL<N>;
+    using L = SL<N>;
     extern __shared__ double2 sm[];
     constexpr int my2 = N / 2 + 1, RSP = RP<N>::RSP;
     double2 *buf = sm, *tws = sm + L::BUF;
@@ -58,14 +58,13 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_sa(Geo g, const doubl
     __syncthreads();
     const int p = blockIdx.x / L::C, rank = blockIdx.x % L::C, nx = g.nx, t = blockIdx.y;
     const int i = p + 1;   // reference plane index
-    const size_t roff = (size_t)rank * L::RL;
-    const TwT tw{tws, N};
+    const size_t roff = (size_t)rank * L::ROWS;
     const double h = sc->heat_ratio, tdx = 2.0 * g.dx, rtdx = 1.0 / tdx;   // reciprocal for qdiv
 #pragma unroll 4
     for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
         const int kz = e / L::PZ, jl = e - kz * L::PZ;
         if (jl == L::MC && rank != 0) continue;
-        const int j = cl_col<N>(jl, rank), ge = kz * my2 + j;
+        const int j = cl_col<L>(jl, rank), ge = kz * my2 + j;
         const double2 c = phi_at(g, phif, i, ge, h);
         double2 f;
         if (t == 0) {
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_sa(Geo g, const doubl
         buf[e] = f;
     }
     __syncthreads();
-    cl_c2r<N>(buf, tw, rank);
+    cl_c2r<L>(buf, tws, rank);
     double *dst;
     if (t == 0) {
         dst = p < nx ? phr + (size_t)p * RSP : phimg;
@@ -114,7 +113,7 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_sa(Geo g, const doubl
             const double *u1 = ubcp + roff;
             const uint8_t *fl = g.fluid + roff;
             double sp = 0.0, su = 0.0, cnt = 0.0;
-            for (int e = threadIdx.x; e < L::RL; e += L::T) {
+            for (int e = threadIdx.x; e < L::ROWS; e += L::T) {
                 if (e % (N + 2) >= N || !fl[e]) continue;
                 sp += u1[e] * b[e];
                 su += u1[e];
@@ -135,10 +134,10 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_sa(Geo g, const doubl
 
 // heat_ratio_new = 1/phim(nx+1), phim = sum(u phi) / (um * count), um = sum(u)/count
 // (nl_allphi.F90:280-301).
-__global__ void k_sheat(Geo g, Scal *sc, const double *spart) {
+__global__ void k_sheat(Geo g, Scal *sc, const double *spart, int parts) {
     if (threadIdx.x != 0 || blockIdx.x != 0 || sc->status) return;
     double sp = 0.0, su = 0.0, cnt = 0.0;
-    for (int r = 0; r < g.plane_ctas; ++r) { sp += spart[r * 3 + 0]; su += spart[r * 3 + 1]; cnt += spart[r * 3 + 2]; }
+    for (int r = 0; r < parts; ++r) { sp += spart[r * 3 + 0]; su += spart[r * 3 + 1]; cnt += spart[r * 3 + 2]; }
     const double um = su / cnt;
     const double phim = sp / (um * cnt);
     sc->heat_ratio_new = 1.0 / phim;
@@ -215,11 +214,11 @@ __global__ void __launch_bounds__(256) k_sflux(Geo g, const double *__restrict__
 // (form_nlphi, nl_allphi.F90:96-114, 190-236; nlphi_graduphi, nlphi.F90:116-128).
 // ============================================================================
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_snl(Geo g, const double *__restrict__ ubcp,
+__global__ void __launch_bounds__(NL<N>::T, NL<N>::MINB) k_snl(Geo g, const double *__restrict__ ubcp,
                                                                const double *__restrict__ phr, const double *__restrict__ dsx,
                                                                double2 *__restrict__ nls, double *__restrict__ nlr,
                                                                Scal *__restrict__ sc) {
-    using L = PL<N>;
+    using L = NL<N>;
     extern __shared__ double2 sm[];
     constexpr int my2 = N / 2 + 1, PS = my2 * N, RSP = RP<N>::RSP;
     double2 *buf = sm, *tws = sm + L::BUF;
@@ -229,8 +228,7 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_snl(Geo g, const doub
     __syncthreads();
     uint32_t phase = 0;
     const int p = blockIdx.x / L::C, rank = blockIdx.x % L::C, nx = g.nx;
-    const size_t roff = (size_t)rank * L::RL;
-    const TwT tw{tws, N};
+    const size_t roff = (size_t)rank * L::ROWS;
     double2 *dst = nls + (size_t)p * PS;
     const double *PB = phr + (size_t)p * RSP + roff;
     for (int q = 0; q < 3; ++q) {
@@ -238,7 +236,7 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_snl(Geo g, const doub
             const double *V = ubcp + ((size_t)(q + 1) * nx + p) * RSP + roff;
             double *b = (double *)buf;
 #pragma unroll 4
-            for (int e = threadIdx.x; e < L::RL; e += L::T) b[e] = V[e] * PB[e];
+            for (int e = threadIdx.x; e < L::ROWS; e += L::T) b[e] = V[e] * PB[e];
             __syncthreads();
         } else {
             if (threadIdx.x == 0) {
@@ -247,76 +245,83 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_snl(Geo g, const doub
             }
             load_wait(&mb, phase, sc);
         }
-        cl_r2c<N>(buf, tw, rank);
-#pragma unroll 4
-        for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
-            const int kz = e / L::PZ, jl = e - kz * L::PZ;
-            if (jl == L::MC && rank != 0) continue;
-            const int j = cl_col<N>(jl, rank), ge = kz * my2 + j;
-            const double2 Xr = cl_unpack<N>(buf, kz, jl, rank);
-            const double2 X = r2c_norm<N>(Xr, g.nrm);
-            if (q == 0) { const double ky = g.ky[j]; dst[ge] = make_double2(-ky * X.y, ky * X.x); }
-            else if (q == 1) { const double kzv = g.kz[kz]; dst[ge] = cadd(dst[ge], make_double2(-kzv * X.y, kzv * X.x)); }
-            else { const double2 a = cadd(dst[ge], X); dst[ge] = make_double2(-a.x, -a.y); }
-        }
+        cl_r2c_out<L>(buf, tws, rank, [&](int kz, int step, int jl, const double2 *X, auto n) {
+            const int j = cl_col<L>(jl, rank), ge = kz * my2 + j;
+            if (q == 0) {
+                const double ky = g.ky[j];
+#pragma unroll
+                for (int k = 0; k < decltype(n)::value; ++k) {
+                    const double2 x = r2c_norm<N>(X[k], g.nrm);
+                    dst[ge + k * step * my2] = make_double2(-ky * x.y, ky * x.x);
+                }
+            } else {
+                update_piece(dst, ge, step * my2, n, [&](int k, double2 d) {
+                    const double2 x = r2c_norm<N>(X[k], g.nrm);
+                    if (q == 1) {
+                        const double kzv = g.kz[kz + k * step];
+                        return cadd(d, make_double2(-kzv * x.y, kzv * x.x));
+                    }
+                    const double2 a = cadd(d, x);
+                    return make_double2(-a.x, -a.y);
+                });
+            }
+        });
         __syncthreads();
     }
-    // c2r of the new nonlinear term (each thread re-reads the values it wrote)
+    // c2r of the new nonlinear term (written by this CTA, above the barrier)
 #pragma unroll 4
     for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
         const int kz = e / L::PZ, jl = e - kz * L::PZ;
         if (jl == L::MC && rank != 0) continue;
-        buf[e] = dst[kz * my2 + cl_col<N>(jl, rank)];
+        buf[e] = dst[kz * my2 + cl_col<L>(jl, rank)];
     }
     __syncthreads();
-    cl_c2r<N>(buf, tw, rank);
+    cl_c2r<L>(buf, tws, rank);
     if (threadIdx.x == 0) { bulk_store(nlr + (size_t)p * RSP + roff, buf, L::RBYTES); bulk_wait_read(); }
 }
 
 // k_simg: real nonlinear term of the image plane nx+1 = c2r(nlphif(1)/heat_ratio)
 // (nl_allphi.F90:219, nlphi.F90:116-128).
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_simg(Geo g, const double2 *__restrict__ nls,
+__global__ void __launch_bounds__(SL<N>::T, SL<N>::MINB) k_simg(Geo g, const double2 *__restrict__ nls,
                                                                 double *__restrict__ nlr, const Scal *__restrict__ sc) {
-    using L = PL<N>;
+    using L = SL<N>;
     extern __shared__ double2 sm[];
     constexpr int my2 = N / 2 + 1, RSP = RP<N>::RSP;
     double2 *buf = sm, *tws = sm + L::BUF;
     load_tw<N>(tws, g);
     const int rank = blockIdx.x % L::C;
-    const TwT tw{tws, N};
     const double h = sc->heat_ratio;
     for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
         const int kz = e / L::PZ, jl = e - kz * L::PZ;
         if (jl == L::MC && rank != 0) continue;
-        const double2 v = nls[kz * my2 + cl_col<N>(jl, rank)];
+        const double2 v = nls[kz * my2 + cl_col<L>(jl, rank)];
         buf[e] = make_double2(v.x / h, v.y / h);
     }
     __syncthreads();
-    cl_c2r<N>(buf, tw, rank);
-    if (threadIdx.x == 0) { bulk_store(nlr + (size_t)g.nx * RSP + (size_t)rank * L::RL, buf, L::RBYTES); bulk_wait_read(); }
+    cl_c2r<L>(buf, tws, rank);
+    if (threadIdx.x == 0) { bulk_store(nlr + (size_t)g.nx * RSP + (size_t)rank * L::ROWS, buf, L::RBYTES); bulk_wait_read(); }
 }
 
 // k_sreal: c2r of spectral planes into the real-field layout of the step
 // (transform order, RSP doubles per plane): restores the real nonlinear term
 // of a restarted scalar (pibm_set_scalar).
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_sreal(Geo g, const double2 *__restrict__ src, double *__restrict__ dst) {
-    using L = PL<N>;
+__global__ void __launch_bounds__(SL<N>::T, SL<N>::MINB) k_sreal(Geo g, const double2 *__restrict__ src, double *__restrict__ dst) {
+    using L = SL<N>;
     extern __shared__ double2 sm[];
     constexpr int my2 = N / 2 + 1, PS = my2 * N, RSP = RP<N>::RSP;
     double2 *buf = sm, *tws = sm + L::BUF;
     load_tw<N>(tws, g);
     const int p = blockIdx.x / L::C, rank = blockIdx.x % L::C;
-    const TwT tw{tws, N};
     for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
         const int kz = e / L::PZ, jl = e - kz * L::PZ;
         if (jl == L::MC && rank != 0) continue;
-        buf[e] = src[(size_t)p * PS + kz * my2 + cl_col<N>(jl, rank)];
+        buf[e] = src[(size_t)p * PS + kz * my2 + cl_col<L>(jl, rank)];
     }
     __syncthreads();
-    cl_c2r<N>(buf, tw, rank);
-    if (threadIdx.x == 0) { bulk_store(dst + (size_t)p * RSP + (size_t)rank * L::RL, buf, L::RBYTES); bulk_wait_read(); }
+    cl_c2r<L>(buf, tws, rank);
+    if (threadIdx.x == 0) { bulk_store(dst + (size_t)p * RSP + (size_t)rank * L::ROWS, buf, L::RBYTES); bulk_wait_read(); }
 }
 
 // ============================================================================
@@ -518,9 +523,9 @@ __global__ void __launch_bounds__(256) k_sspread(Geo g, const double *__restrict
 
 // k_sff: ffphi = r2c(fr) over planes 1..nx (bcsetscal, bc_scalar.F90:323-349).
 template <int N>
-__global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_sff(Geo g, const double *__restrict__ sfr, double2 *__restrict__ ffs,
+__global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) k_sff(Geo g, const double *__restrict__ sfr, double2 *__restrict__ ffs,
                                                                Scal *__restrict__ sc) {
-    using L = PL<N>;
+    using L = RL<N>;
     extern __shared__ double2 sm[];
     constexpr int my2 = N / 2 + 1, PS = my2 * N, RSP = RP<N>::RSP;
     double2 *buf = sm, *tws = sm + L::BUF;
@@ -530,21 +535,17 @@ __global__ void __launch_bounds__(PL<N>::T, PL<N>::MINB) k_sff(Geo g, const doub
     __syncthreads();
     uint32_t phase = 0;
     const int p = blockIdx.x / L::C, rank = blockIdx.x % L::C;
-    const TwT tw{tws, N};
     if (threadIdx.x == 0) {
         fence_async_smem();
-        bulk_load(buf, sfr + (size_t)p * RSP + (size_t)rank * L::RL, L::RBYTES, &mb);
+        bulk_load(buf, sfr + (size_t)p * RSP + (size_t)rank * L::ROWS, L::RBYTES, &mb);
     }
     load_wait(&mb, phase, sc);
-    cl_r2c<N>(buf, tw, rank);
     double2 *dst = ffs + (size_t)p * PS;
-#pragma unroll 4
-    for (int e = threadIdx.x; e < L::NOUT; e += L::T) {
-        const int kz = e / L::PZ, jl = e - kz * L::PZ;
-        if (jl == L::MC && rank != 0) continue;
-        const double2 X = cl_unpack<N>(buf, kz, jl, rank);
-        dst[kz * my2 + cl_col<N>(jl, rank)] = r2c_norm<N>(X, g.nrm);
-    }
+    cl_r2c_out<L>(buf, tws, rank, [&](int kz, int step, int jl, const double2 *X, auto n) {
+        double2 *d = dst + kz * my2 + cl_col<L>(jl, rank);
+#pragma unroll
+        for (int k = 0; k < decltype(n)::value; ++k) d[k * step * my2] = r2c_norm<N>(X[k], g.nrm);
+    });
 }
 
 // ============================================================================
@@ -711,13 +712,13 @@ int moving_scalar_kernels_per_step();
 template <int N>
 static void enqueue_scalar_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s) {
     const int old = 1 - cur;
-    launch_planes<N>(k_sa<N>, g.nx + 1, 5, s, g, (const double2 *)b.phif, (const double *)b.ubcp, b.phr, b.phimg,
+    launch_planes<SL<N>>(k_sa<N>, g.nx + 1, 5, s, g, (const double2 *)b.phif, (const double *)b.ubcp, b.phr, b.phimg,
                      b.sdf, b.gph, (const Scal *)b.sc, b.spart);
-    k_sheat<<<1, 32, 0, s>>>(g, b.sc, b.spart);
+    k_sheat<<<1, 32, 0, s>>>(g, b.sc, b.spart, SL<N>::C);
     k_sflux<N><<<(RP<N>::RSP * ((g.nx + kScalarFluxSeg - 1) / kScalarFluxSeg) + 255) / 256, 256, 0, s>>>(g, b.ubcp, b.phr, b.phimg, b.dsx, b.sc);
-    launch_planes<N>(k_snl<N>, g.nx, 1, s, g, (const double *)b.ubcp, (const double *)b.phr, (const double *)b.dsx,
+    launch_planes<NL<N>>(k_snl<N>, g.nx, 1, s, g, (const double *)b.ubcp, (const double *)b.phr, (const double *)b.dsx,
                      b.nls[cur], b.nlr[cur], b.sc);
-    launch_planes<N>(k_simg<N>, 1, 1, s, g, (const double2 *)b.nls[cur], b.nlr[cur], (const Scal *)b.sc);
+    launch_planes<SL<N>>(k_simg<N>, 1, 1, s, g, (const double2 *)b.nls[cur], b.nlr[cur], (const Scal *)b.sc);
     if (g.nbody > 0) k_sbnd<N><<<g.nbody * kDragSplit, 256, 0, s>>>(g, b.gph, b.sc, b.sdpart);
     if (g.moving) enqueue_moving_scalar(g, b.mov, b.sc, s);
     if (g.nsev > 0) {
@@ -725,7 +726,7 @@ static void enqueue_scalar_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s) 
         if (g.moving) enqueue_sspread_dyn(g, b.mov, b.sctb, b.sfd, b.sfr, b.sc, s);
         else if (g.ssp_nnodes > 0) k_sspread<<<(g.ssp_nnodes + 255) / 256, 256, 0, s>>>(g, b.sctb, b.sfd, b.sfr, b.sc);
     }
-    launch_planes<N>(k_sff<N>, g.nx, 1, s, g, (const double *)b.sfr, b.ffs, b.sc);
+    launch_planes<RL<N>>(k_sff<N>, g.nx, 1, s, g, (const double *)b.sfr, b.ffs, b.sc);
     constexpr int LT = SLinesCfg<N>::LT;
     k_slines<N, LT><<<(g.PS + LT - 1) / LT, LT * 32, slines_smem<N>(), s>>>(g, b.phif, b.nls[cur], b.nls[old], b.ffs, b.sc);
     k_sfin<<<1, 256, 0, s>>>(g, b.sc, b.sdpart, b.flux_body);
@@ -743,7 +744,7 @@ void enqueue_scalar(const Geo &g, DevBufs &b, int cur, cudaStream_t s) {
 
 template <int N>
 static void enqueue_scalar_c2r_t(const Geo &g, const double2 *src, double *dst, int nplanes, cudaStream_t s) {
-    launch_planes<N>(k_sreal<N>, nplanes, 1, s, g, src, dst);
+    launch_planes<SL<N>>(k_sreal<N>, nplanes, 1, s, g, src, dst);
 }
 // c2r of nplanes spectral planes into the step's real layout.
 void enqueue_scalar_c2r(const Geo &g, const double2 *src, double *dst, int nplanes, cudaStream_t s) {
@@ -767,13 +768,13 @@ int scalar_kernels_per_step(const Geo &g) {
 
 template <int N>
 static cudaError_t set_scalar_attrs() {
-    const int maxs = (int)plane_smem<N>();
+    const int maxs = (int)PL<N>::SMEM;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(k_sa<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_snl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_simg<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_sreal<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_sff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_sa<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SL<N>::SMEM)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_snl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NL<N>::SMEM)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_simg<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SL<N>::SMEM)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_sreal<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SL<N>::SMEM)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_sff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_slines<N, SLinesCfg<N>::LT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slines_smem<N>());
 }
 

@@ -51,6 +51,22 @@ template <int N> __device__ __forceinline__ double2 r2c_norm(double2 x, double n
 // may set the word while the block starts.  Call with every thread present.
 __device__ __forceinline__ bool block_failed(const Scal *sc) { return __syncthreads_or(sc->status != 0) != 0; }
 
+// Start the copy of a spectral plane src[kz][ky] into the CTA's column-phase
+// buffer (completes on mb): the whole plane is one bulk copy when the CTA
+// holds it alone; else the CTA's MC columns of every kz row as N bulk copies
+// into the padded rows, and rank 0's Nyquist column (slot MC) with plain loads.
+template <class L>
+__device__ __forceinline__ void load_plane(double2 *buf, const double2 *__restrict__ src, int rank, uint64_t *mb) {
+    constexpr int my2 = L::N / 2 + 1;
+    if constexpr (L::C == 1) {
+        if (threadIdx.x == 0) bulk_load(buf, src, L::N * my2 * 16, mb);
+    } else {
+        if (threadIdx.x < 32) bulk_load_rows(buf, L::PZ * 16, src + rank * L::MC, (size_t)my2 * 16, L::MC * 16, L::N, mb);
+        if (rank == 0)
+            for (int kz = threadIdx.x; kz < L::N; kz += L::T) buf[kz * L::PZ + L::MC] = src[kz * my2 + L::M];
+    }
+}
+
 // Bounded wait on the CTA's load barrier; records a timeout in the status word.
 __device__ __forceinline__ void load_wait(uint64_t *mb, uint32_t &phase, Scal *sc) {
     if (!mbar_wait(mb, phase)) atomicCAS(&sc->status, 0, PIBM_ERR_TIMEOUT);
@@ -207,22 +223,19 @@ __device__ __forceinline__ double dot_ijk(const Sten &s, const double *f) {
 // ============================================================================
 // Plane-kernel launches
 // ============================================================================
-template <int N>
-inline size_t plane_smem() { return cl_smem<N>(); }
-
-// Launch a plane kernel on nplanes planes: PL<N>::C CTAs per plane, grouped
+// Launch a plane kernel on nplanes planes: L::C CTAs per plane, grouped
 // into clusters of that size (the plane's CTAs exchange data through
 // distributed shared memory).
-template <int N, typename... KArgs, typename... Args>
+template <class L, typename... KArgs, typename... Args>
 inline void launch_planes(void (*k)(KArgs...), int nplanes, int items, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(nplanes * PL<N>::C), (unsigned)items, 1);
-    cfg.blockDim = dim3(PL<N>::T, 1, 1);
-    cfg.dynamicSmemBytes = plane_smem<N>();
+    cfg.gridDim = dim3((unsigned)(nplanes * L::C), (unsigned)items, 1);
+    cfg.blockDim = dim3(L::T, 1, 1);
+    cfg.dynamicSmemBytes = L::SMEM;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = PL<N>::C;
+    at[0].val.clusterDim.x = L::C;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
@@ -236,16 +249,16 @@ inline void launch_planes(void (*k)(KArgs...), int nplanes, int items, cudaStrea
 constexpr int kScalarFluxSeg = 32;
 
 // launch_planes for a fused batch: nz runs of the same size along gridDim.z.
-template <int N, typename... KArgs, typename... Args>
+template <class L, typename... KArgs, typename... Args>
 inline void launch_planes_z(void (*k)(KArgs...), int nplanes, int items, int nz, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(nplanes * PL<N>::C), (unsigned)items, (unsigned)nz);
-    cfg.blockDim = dim3(PL<N>::T, 1, 1);
-    cfg.dynamicSmemBytes = plane_smem<N>();
+    cfg.gridDim = dim3((unsigned)(nplanes * L::C), (unsigned)items, (unsigned)nz);
+    cfg.blockDim = dim3(L::T, 1, 1);
+    cfg.dynamicSmemBytes = L::SMEM;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = PL<N>::C;
+    at[0].val.clusterDim.x = L::C;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;

@@ -56,6 +56,28 @@ def test_noalloc_ff2cr_matches_allocating_entry_point():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [32, 64, 96, 128])
+def test_noalloc_ff2cr_output_aligned_to_doubles_only(n):
+    """A real output buffer at an odd multiple of 8 bytes takes the narrow
+    stores: bitwise the values of the wide ones, nothing written outside."""
+    import torch
+
+    lib = pk.load_library()
+    a = _spectral_planes(np.random.default_rng(n), 2, n)
+    d_a = torch.from_numpy(a.view(np.float64).copy()).cuda()
+    size = 2 * n * n
+    out = [torch.full((size + 2,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(2)]
+    for k, d_b in enumerate(out):
+        rc = lib.pibm_ff2cr_noalloc(n, n, 2, C.c_void_p(d_a.data_ptr()), C.c_void_p(d_b.data_ptr() + 8 * k),
+                                    C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0, lib.pibm_last_error().decode()
+    torch.cuda.synchronize()
+    wide, narrow = out[0].cpu().numpy(), out[1].cpu().numpy()
+    assert np.array_equal(wide[:size], narrow[1:size + 1])
+    assert np.isnan(wide[size:]).all() and np.isnan(narrow[0]) and np.isnan(narrow[size + 1])
+
+
+@pytest.mark.gpu
 def test_noalloc_ff2cr_rejects_sizes_beyond_the_static_scratch():
     import torch
 
