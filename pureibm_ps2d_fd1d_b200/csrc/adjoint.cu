@@ -75,24 +75,15 @@ __global__ void __launch_bounds__(LT * 32) k_adj_lines(Geo g, const double2 *__r
     constexpr int R = NX / 32;
     constexpr int NP = lines_pitch<NX, LT>();
     extern __shared__ double2 sm[];
-    double2 *tws = sm;
-    double2 *D = tws + NX;                 // lambda d, then lambda of the divcorr right-hand side
+    double2 *D = sm;                       // lambda d, then lambda of the divcorr right-hand side
     double2 *P = D + LT * NP;              // lambda P, then lambda of the pressure right-hand side
     double2 *U = P + LT * NP;              // [comp][line][i]: lambda u_n -> lambda Us -> lambda r
-    double *gam = (double *)(U + 3 * LT * NP);
-    double2 *st = (double2 *)(gam + NX);
-    double *lcs = (double *)(st + 32);        // per-lane constants of the solves
-    double2 *ltr = (double2 *)(lcs + NX);
-    for (int t = threadIdx.x; t < NX; t += blockDim.x) tws[t] = g.tw[t];
-    fill_stage_table<32>(st, g.tw, NX);
-    fill_line_tw<R>(lcs, ltr, g.tw);
     const int PS = g.PS, nx = NX;
     const int q0 = blockIdx.x * LT;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const double dx = g.dx, dx2 = g.dx2, dt = sc->dt, vis = g.vis, rdx2 = 1.0 / dx2;
     const double c1 = g.c1, c2 = g.c2, c3 = g.c3, c4 = g.c4;
     const double alp = (c1 + c2) * dt, c2dtv = (c2 * dt) * vis, gd = dt * vis * c1;
-    const LineTw<R> tw{{tws, NX, 1, st}, lcs, ltr};
     auto KY = [&](int q) { return g.ky[q % g.my2]; };
     auto KZ = [&](int q) { return g.kz[q / g.my2]; };
     auto W = [&](int i) { return i < 0 ? i + nx : (i >= nx ? i - nx : i); };
@@ -100,8 +91,8 @@ __global__ void __launch_bounds__(LT * 32) k_adj_lines(Geo g, const double2 *__r
     for (int t = threadIdx.x; t < LT * NX; t += blockDim.x) {
         const int line = t % LT, i = t / LT, q = q0 + line;
         const bool in = q < PS;
-        for (int n = 0; n < 3; ++n) U[(n * LT + line) * NP + i] = in ? lu[((size_t)n * nx + i) * PS + q] : make_double2(0.0, 0.0);
-        P[line * NP + i] = in ? lp[(size_t)i * PS + q] : make_double2(0.0, 0.0);
+        for (int n = 0; n < 3; ++n) U[(n * LT + line) * NP + row_slot(i)] = in ? lu[((size_t)n * nx + i) * PS + q] : make_double2(0.0, 0.0);
+        P[line * NP + row_slot(i)] = in ? lp[(size_t)i * PS + q] : make_double2(0.0, 0.0);
     }
     __syncthreads();
     // ---- divcorr^T: lambda d ----
@@ -109,31 +100,26 @@ __global__ void __launch_bounds__(LT * 32) k_adj_lines(Geo g, const double2 *__r
         const int line = t % LT, i = t / LT, q = min(q0 + line, PS - 1);
         const double ky = KY(q), kz = KZ(q), w2 = g.w2[q];
         const double2 *Pl = P + line * NP, *U0 = U + (0 * LT + line) * NP, *U1 = U + (1 * LT + line) * NP, *U2 = U + (2 * LT + line) * NP;
-        const double2 pm = Pl[W(i - 1)], p0 = Pl[i], pp = Pl[W(i + 1)];
+        const double2 pm = Pl[row_slot(W(i - 1))], p0 = Pl[row_slot(i)], pp = Pl[row_slot(W(i + 1))];
         double2 v = make_double2(p0.x - c2dtv * (qdiv((pm.x - 2.0 * p0.x) + pp.x, dx2, rdx2) - w2 * p0.x),
                                  p0.y - c2dtv * (qdiv((pm.y - 2.0 * p0.y) + pp.y, dx2, rdx2) - w2 * p0.y));
-        const double2 a0 = U0[i], a1 = U0[W(i + 1)];
+        const double2 a0 = U0[row_slot(i)], a1 = U0[row_slot(W(i + 1))];
         v = make_double2(v.x - (alp / dx) * (a0.x - a1.x), v.y - (alp / dx) * (a0.y - a1.y));
         // conj(-alp wy / 2) = i alp ky / 2
-        v = cadd(v, mul_is(cadd(U1[i], U1[W(i + 1)]), 0.5 * alp * ky));
-        v = cadd(v, mul_is(cadd(U2[i], U2[W(i + 1)]), 0.5 * alp * kz));
-        D[line * NP + i] = v;
+        v = cadd(v, mul_is(cadd(U1[row_slot(i)], U1[row_slot(W(i + 1))]), 0.5 * alp * ky));
+        v = cadd(v, mul_is(cadd(U2[row_slot(i)], U2[row_slot(W(i + 1))]), 0.5 * alp * kz));
+        D[line * NP + row_slot(i)] = v;
     }
     __syncthreads();
     const int qw = q0 + w;
     const bool wact = qw < PS;
     const double w2w = wact ? g.w2[qw] : 0.0;
-    bool ok = true;
     {
-        const double a = 1.0 / dx2 - 0.25 * w2w, bd = -2.0 / dx2 - 0.5 * w2w, c = 1.0 / dx2 - 0.25 * w2w;
+        const double a = 1.0 / dx2 - 0.25 * w2w, bd = -2.0 / dx2 - 0.5 * w2w;
         double2 *row = D + w * NP;
         if (wact) {
-            if (qw == 0) {
-                if (lane == 0) ok = thomas_real(row, gam, a, bd, c, NX - 1) && ok;
-                __syncwarp();
-            } else {
-                circulant_solve<R>(row, a, bd, tw, lane);
-            }
+            if (qw == 0) dirichlet_solve_row<R>(row, a, lane);
+            else circ_solve_row<R>(row, circ_factor<R>(a, bd), lane);
         }
     }
     __syncthreads();
@@ -141,19 +127,20 @@ __global__ void __launch_bounds__(LT * 32) k_adj_lines(Geo g, const double2 *__r
     for (int t = threadIdx.x; t < LT * NX; t += blockDim.x) {
         const int line = t % LT, i = t / LT, q = min(q0 + line, PS - 1);
         const double ky = KY(q), kz = KZ(q);
-        const double2 dm = D[line * NP + W(i - 1)], d0 = D[line * NP + i];
+        const double2 dm = D[line * NP + row_slot(W(i - 1))], d0 = D[line * NP + row_slot(i)];
         double2 *U0 = U + (0 * LT + line) * NP, *U1 = U + (1 * LT + line) * NP, *U2 = U + (2 * LT + line) * NP;
-        U0[i] = make_double2(U0[i].x + (dm.x - d0.x) / (dx * alp), U0[i].y + (dm.y - d0.y) / (dx * alp));
+        U0[row_slot(i)] = make_double2(U0[row_slot(i)].x + (dm.x - d0.x) / (dx * alp), U0[row_slot(i)].y + (dm.y - d0.y) / (dx * alp));
         // conj(0.5 wy / alp) = -i 0.5 ky / alp
-        U1[i] = cadd(U1[i], mul_cis(cadd(d0, dm), 0.5 * ky / alp));
-        U2[i] = cadd(U2[i], mul_cis(cadd(d0, dm), 0.5 * kz / alp));
+        U1[row_slot(i)] = cadd(U1[row_slot(i)], mul_cis(cadd(d0, dm), 0.5 * ky / alp));
+        U2[row_slot(i)] = cadd(U2[row_slot(i)], mul_cis(cadd(d0, dm), 0.5 * kz / alp));
     }
     __syncthreads();
     // ---- ustep^T: lambda r = A_u^-1 lambda Us per component ----
     if (wact) {
         const double a = -(1.0 * dt * vis * c2 / dx2);
         const double bd = 1.0 + dt * vis * c2 * (1.0 * 2.0 / dx2 + w2w);
-        for (int n = 0; n < 3; ++n) circulant_solve<R>(U + (n * LT + w) * NP, a, bd, tw, lane);
+        const Circ<R> ku = circ_factor<R>(a, bd);
+        for (int n = 0; n < 3; ++n) circ_solve_row<R>(U + (n * LT + w) * NP, ku, lane);
     }
     __syncthreads();
     // lambda P += (grad P in the ustep right-hand sides)^T; lambda u_{n-1} (ustep part)
@@ -164,17 +151,17 @@ __global__ void __launch_bounds__(LT * 32) k_adj_lines(Geo g, const double2 *__r
         const double fy = 1.0 - dt * vis * c1 * w2;
         const double2 *R0 = U + (0 * LT + line) * NP, *R1 = U + (1 * LT + line) * NP, *R2 = U + (2 * LT + line) * NP;
         const int ip = W(i + 1), im = W(i - 1);
-        double2 v = P[line * NP + i];
-        v = make_double2(v.x - (alp / dx) * (R0[i].x - R0[ip].x), v.y - (alp / dx) * (R0[i].y - R0[ip].y));
+        double2 v = P[line * NP + row_slot(i)];
+        v = make_double2(v.x - (alp / dx) * (R0[row_slot(i)].x - R0[row_slot(ip)].x), v.y - (alp / dx) * (R0[row_slot(i)].y - R0[row_slot(ip)].y));
         // -conj(alp/2 wy) = i alp ky / 2
-        v = cadd(v, mul_is(cadd(R1[i], R1[ip]), 0.5 * alp * ky));
-        v = cadd(v, mul_is(cadd(R2[i], R2[ip]), 0.5 * alp * kz));
-        P[line * NP + i] = v;
+        v = cadd(v, mul_is(cadd(R1[row_slot(i)], R1[row_slot(ip)]), 0.5 * alp * ky));
+        v = cadd(v, mul_is(cadd(R2[row_slot(i)], R2[row_slot(ip)]), 0.5 * alp * kz));
+        P[line * NP + row_slot(i)] = v;
         if (q < PS) {
             const double2 *Rn[3] = {R0, R1, R2};
 #pragma unroll
             for (int n = 0; n < 3; ++n) {
-                const double2 r0 = Rn[n][i], rm = Rn[n][im], rp = Rn[n][ip];
+                const double2 r0 = Rn[n][row_slot(i)], rm = Rn[n][row_slot(im)], rp = Rn[n][row_slot(ip)];
                 lu2[((size_t)n * nx + i) * PS + q] = make_double2(fy * r0.x + qdiv(gd * ((rm.x + rp.x) - 2.0 * r0.x), dx2, rdx2),
                                                                  fy * r0.y + qdiv(gd * ((rm.y + rp.y) - 2.0 * r0.y), dx2, rdx2));
             }
@@ -183,15 +170,11 @@ __global__ void __launch_bounds__(LT * 32) k_adj_lines(Geo g, const double2 *__r
     __syncthreads();
     // ---- pressure^T: lambda S = A_p^-1 lambda P / (c1 + c2) ----
     {
-        const double a = 1.0 / dx2 - 0.25 * w2w, bd = -2.0 / dx2 - 0.5 * w2w, c = 1.0 / dx2 - 0.25 * w2w;
+        const double a = 1.0 / dx2 - 0.25 * w2w, bd = -2.0 / dx2 - 0.5 * w2w;
         double2 *row = P + w * NP;
         if (wact) {
-            if (qw == 0) {
-                if (lane == 0) ok = thomas_real(row, gam, a, bd, c, NX - 1) && ok;
-                __syncwarp();
-            } else {
-                circulant_solve<R>(row, a, bd, tw, lane);
-            }
+            if (qw == 0) dirichlet_solve_row<R>(row, a, lane);
+            else circ_solve_row<R>(row, circ_factor<R>(a, bd), lane);
         }
     }
     __syncthreads();
@@ -201,11 +184,11 @@ __global__ void __launch_bounds__(LT * 32) k_adj_lines(Geo g, const double2 *__r
         if (q >= PS) continue;
         const double ky = KY(q), kz = KZ(q);
         const double cs = 1.0 / (c1 + c2);
-        const double2 s0 = cscale(P[line * NP + i], cs), sm = cscale(P[line * NP + W(i - 1)], cs);
+        const double2 s0 = cscale(P[line * NP + row_slot(i)], cs), sm = cscale(P[line * NP + row_slot(W(i - 1))], cs);
         const double2 dif = csub(sm, s0), sum = cadd(s0, sm);
 #pragma unroll
         for (int n = 0; n < 3; ++n) {
-            const double2 r = U[(n * LT + line) * NP + i];
+            const double2 r = U[(n * LT + line) * NP + row_slot(i)];
             double2 bnl, bff, bon;
             if (n == 0) { bnl = cscale(dif, c3 / dx); bff = cscale(dif, 1.0 / dx); bon = cscale(dif, c4 / dx); }
             else {
@@ -219,13 +202,12 @@ __global__ void __launch_bounds__(LT * 32) k_adj_lines(Geo g, const double2 *__r
         }
         lp2[(size_t)i * PS + q] = make_double2(0.0, 0.0);
     }
-    if (!ok) atomicCAS(&as->status, 0, PIBM_ERR_PIVOT);
 }
 
 template <int NX>
 static size_t adj_lines_smem() {
     constexpr int LT = NX >= 256 ? 4 : 8;
-    return (size_t)(NX + 5 * LT * lines_pitch<NX, LT>() + 32) * sizeof(double2) + NX * sizeof(double) + line_tw_bytes<NX / 32>();
+    return (size_t)(5 * LT * lines_pitch<NX, LT>()) * sizeof(double2);
 }
 
 // ============================================================================

@@ -836,15 +836,9 @@ __global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) k_ff(Geo g, const doubl
 // (poisson.F90:55-508, usteptime.F90:45-269, check_divergence
 // steptheflow.F90:219-240).
 //
-// Every cyclic system of velstep has constant coefficients (a = c, b on every
-// row, periodic coupling), i.e. it is a symmetric circulant matrix; the
-// reference solves it with Thomas + Sherman-Morrison (tridiagonal.F90:90-150,
-// usteptime.F90:344-349,457-468).  Here one warp solves one line exactly
-// through its eigen-decomposition: forward FFT along x in registers
-// (group_fft), division by N*lambda_m with lambda_m = b + 2a cos(2 pi m/N),
-// and the exact inverse of the forward stages.  The (ky,kz) = (0,0) line is
-// not circulant (nx-1 unknowns, p(nx) = 0: poisson.F90:127-142, 309-325) and
-// keeps the reference's Thomas recursion.
+// One warp solves one line (line_solve.cuh): two cyclic first-order recurrences
+// over blocks of R consecutive planes, the (ky,kz) = (0,0) pressure line by
+// its Green's function.
 // Tiles live in shared memory as [line][i]; global loads and stores run over
 // consecutive lines (contiguous in the [i][k][j] layout).
 // ============================================================================
@@ -855,32 +849,22 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
     constexpr int R = NX / 32;
     constexpr int NP = lines_pitch<NX, LT>();
     extern __shared__ double2 sm[];
-    double2 *tws = sm;
-    double2 *RHS = tws + NX;
+    double2 *RHS = sm;
     double2 *P = RHS + LT * NP;
     double2 *U = P + LT * NP;                 // [comp][line][i]
-    double *gam = (double *)(U + 3 * LT * NP);
-    double2 *st = (double2 *)(gam + NX);      // cross-lane stage twiddles
-    double *lcs = (double *)(st + 32);        // per-lane constants of the solves
-    double2 *ltr = (double2 *)(lcs + NX);
     if (block_failed(sc)) return;
-    for (int t = threadIdx.x; t < NX; t += blockDim.x) tws[t] = g.tw[t];
-    fill_stage_table<32>(st, g.tw, NX);
-    fill_line_tw<R>(lcs, ltr, g.tw);
     const int PS = g.PS, nx = NX;
     const int q0 = blockIdx.x * LT;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const double dx = g.dx, dx2 = g.dx2, dt = sc->dt, vis = g.vis;
     const double c1 = g.c1, c2 = g.c2, c3 = g.c3, c4 = g.c4;
     const double c12 = c1 + c2, rdx = 1.0 / dx, rdx2 = 1.0 / dx2, rc12 = 1.0 / c12;   // divisors and reciprocals for qdiv
-    const LineTw<R> tw{{tws, NX, 1, st}, lcs, ltr};
     auto KY = [&](int q) { return g.ky[q % g.my2]; };
     auto KZ = [&](int q) { return g.kz[q / g.my2]; };
     auto G = [&](const double2 *f, int comp, int i, int q) -> double2 {
         i = i >= nx ? i - nx : (i < 0 ? i + nx : i);
         return f[((size_t)comp * nx + i) * PS + q];
     };
-    bool ok = true;
     // ---------------- pressure: source (poisson.F90:97-116) and old p ----------------
     // Thread t holds (line t % LT, plane t / LT): for LT = 8 the plane i+1 of a lane
     // sits LT lanes higher in the same warp, except in the warp's last plane row.
@@ -912,13 +896,13 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
         }
 #pragma unroll
         for (int n = 0; n < 3; ++n) tt = cadd_rn(tt, psrc_term<true>(n, c4, x0[6 + n], x1[6 + n], ky, kz, dx, rdx));
-        RHS[line * NP + i] = make_double2(qdiv(tt.x, c12, rc12), qdiv(tt.y, c12, rc12));
-        P[line * NP + i] = p[(size_t)i * PS + q];
+        RHS[line * NP + row_slot(i)] = make_double2(qdiv(tt.x, c12, rc12), qdiv(tt.y, c12, rc12));
+        P[line * NP + row_slot(i)] = p[(size_t)i * PS + q];
         // explicit part of the ustep right-hand sides, dt*(c3 nl + ff + c4 onl) per component
         // (usteptime.F90:291-297), kept in the velocity tiles until each component is solved
 #pragma unroll
         for (int n = 0; n < 3; ++n)
-            U[(n * LT + line) * NP + i] = cadd_rn(cadd_rn(cscale_rn(x0[n], dt * c3), cscale_rn(x0[3 + n], dt)), cscale_rn(x0[6 + n], dt * c4));
+            U[(n * LT + line) * NP + row_slot(i)] = cadd_rn(cadd_rn(cscale_rn(x0[n], dt * c3), cscale_rn(x0[3 + n], dt)), cscale_rn(x0[6 + n], dt * c4));
     }
     __syncthreads();
     const int qw = q0 + w;
@@ -928,28 +912,25 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
     {
         double2 *row = RHS + w * NP;
         if (wact) {
-            if (qw == 0) {
-                if (lane == 0) ok = thomas_real(row, gam, kw.pa, kw.pb, kw.pc, NX - 1) && ok;
-                __syncwarp();
-            } else {
-                circulant_solve<R>(row, kw.pa, kw.pb, tw, lane);
-            }
+            if (qw == 0) dirichlet_solve_row<R>(row, kw.pa, lane);
+            else circ_solve_row<R>(row, circ_factor<R>(kw.pa, kw.pb), lane);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const int i = lane + 32 * r;
-                P[w * NP + i] = p_update(P[w * NP + i], row[i]);
+                P[w * NP + row_slot(i)] = p_update(P[w * NP + row_slot(i)], row[row_slot(i)]);
             }
         }
     }
     __syncthreads();
     // ---------------- ustep per component (usteptime.F90:73-470) ----------------
     constexpr int EPT = (LT * NX) / (LT * 32);   // tile elements per thread
+    const Circ<R> ku = circ_factor<R>(kw.ua, kw.ub);
     for (int n = 0; n < 3; ++n) {
         // stage u_n of the tile, then form every right-hand side from the staged
         // neighbours before overwriting the tile with them
         for (int t = threadIdx.x; t < LT * NX; t += blockDim.x) {
             const int line = t % LT, i = t / LT, q = q0 + line;
-            RHS[line * NP + i] = q < PS ? G(u, n, i, q) : make_double2(0.0, 0.0);
+            RHS[line * NP + row_slot(i)] = q < PS ? G(u, n, i, q) : make_double2(0.0, 0.0);
         }
         __syncthreads();
         double2 rr[EPT];
@@ -960,22 +941,22 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
             if (q >= PS) continue;
             const LineCoef kq = line_coef(dt, vis, c1, c2, dx2, g.w2[q]);
             const int im = i == 0 ? nx - 1 : i - 1, ip = i == nx - 1 ? 0 : i + 1;
-            rr[k] = ustep_rhs(n, kq, RHS[line * NP + i], RHS[line * NP + im], RHS[line * NP + ip], U[(n * LT + line) * NP + i],
-                              P[line * NP + im], P[line * NP + i], i == 0, KY(q), KZ(q), dx, rdx, dx2, rdx2);
+            rr[k] = ustep_rhs(n, kq, RHS[line * NP + row_slot(i)], RHS[line * NP + row_slot(im)], RHS[line * NP + row_slot(ip)], U[(n * LT + line) * NP + row_slot(i)],
+                              P[line * NP + row_slot(im)], P[line * NP + row_slot(i)], i == 0, KY(q), KZ(q), dx, rdx, dx2, rdx2);
         }
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < EPT; ++k) {
             const int t = threadIdx.x + k * LT * 32;
             const int line = t % LT, i = t / LT, q = q0 + line;
-            if (q < PS) RHS[line * NP + i] = rr[k];
+            if (q < PS) RHS[line * NP + row_slot(i)] = rr[k];
         }
         __syncthreads();
         if (wact) {
             double2 *row = RHS + w * NP;
-            circulant_solve<R>(row, kw.ua, kw.ub, tw, lane);
+            circ_solve_row<R>(row, ku, lane);
 #pragma unroll
-            for (int r = 0; r < R; ++r) U[(n * LT + w) * NP + lane + 32 * r] = row[lane + 32 * r];
+            for (int r = 0; r < R; ++r) U[(n * LT + w) * NP + row_slot(lane + 32 * r)] = row[row_slot(lane + 32 * r)];
         }
         __syncthreads();
     }
@@ -986,19 +967,15 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
         if (q >= PS) continue;
         const int ip = i == nx - 1 ? 0 : i + 1;
         const double2 *U1 = U + (0 * LT + line) * NP, *U2 = U + (1 * LT + line) * NP, *U3 = U + (2 * LT + line) * NP;
-        const double2 tt = div_term(U1[i], U1[ip], U2[i], U2[ip], U3[i], U3[ip], KY(q), KZ(q), dx, rdx);
-        RHS[line * NP + i] = make_double2(qdiv(tt.x, alpc, ralpc), qdiv(tt.y, alpc, ralpc));
+        const double2 tt = div_term(U1[row_slot(i)], U1[row_slot(ip)], U2[row_slot(i)], U2[row_slot(ip)], U3[row_slot(i)], U3[row_slot(ip)], KY(q), KZ(q), dx, rdx);
+        RHS[line * NP + row_slot(i)] = make_double2(qdiv(tt.x, alpc, ralpc), qdiv(tt.y, alpc, ralpc));
     }
     __syncthreads();
     if (wact) {
         const double ky = KY(qw), kz = KZ(qw);
         double2 *row = RHS + w * NP;
-        if (qw == 0) {
-            if (lane == 0) ok = thomas_real(row, gam, kw.pa, kw.pb, kw.pc, NX - 1) && ok;
-            __syncwarp();
-        } else {
-            circulant_solve<R>(row, kw.pa, kw.pb, tw, lane);
-        }
+        if (qw == 0) dirichlet_solve_row<R>(row, kw.pa, lane);
+        else circ_solve_row<R>(row, circ_factor<R>(kw.pa, kw.pb), lane);
         double2 *U1 = U + (0 * LT + w) * NP, *U2 = U + (1 * LT + w) * NP, *U3 = U + (2 * LT + w) * NP;
         double2 *Pw = P + w * NP;
         double2 nu1[R], nu2[R], nu3[R], np[R];
@@ -1006,14 +983,14 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
         for (int r = 0; r < R; ++r) {
             const int i = lane + 32 * r;
             const int im = i == 0 ? nx - 1 : i - 1, ip = i == nx - 1 ? 0 : i + 1;
-            divcorr_update(kw, row[i], row[im], row[ip], i == 0, U1[i], U2[i], U3[i], Pw[i], ky, kz, w2w, dx, rdx, dx2, rdx2, nu1[r],
+            divcorr_update(kw, row[row_slot(i)], row[row_slot(im)], row[row_slot(ip)], i == 0, U1[row_slot(i)], U2[row_slot(i)], U3[row_slot(i)], Pw[row_slot(i)], ky, kz, w2w, dx, rdx, dx2, rdx2, nu1[r],
                            nu2[r], nu3[r], np[r]);
         }
         __syncwarp();
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int i = lane + 32 * r;
-            U1[i] = nu1[r]; U2[i] = nu2[r]; U3[i] = nu3[r]; Pw[i] = np[r];
+            U1[row_slot(i)] = nu1[r]; U2[row_slot(i)] = nu2[r]; U3[row_slot(i)] = nu3[r]; Pw[row_slot(i)] = np[r];
         }
         __syncwarp();
         // check_divergence for this line
@@ -1021,7 +998,7 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int i = lane + 32 * r, ip = i == nx - 1 ? 0 : i + 1;
-            dmax = fmax(dmax, cabs_rn(div_term(U1[i], U1[ip], U2[i], U2[ip], U3[i], U3[ip], ky, kz, dx, rdx)));
+            dmax = fmax(dmax, cabs_rn(div_term(U1[row_slot(i)], U1[row_slot(ip)], U2[row_slot(i)], U2[row_slot(ip)], U3[row_slot(i)], U3[row_slot(ip)], ky, kz, dx, rdx)));
         }
         for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
         if (lane == 0) atomicMax(&sc->divmax_bits, (unsigned long long)__double_as_longlong(dmax));
@@ -1032,10 +1009,9 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
         const int line = t % LT, i = t / LT, q = q0 + line;
         if (q >= PS) continue;
 #pragma unroll
-        for (int n = 0; n < 3; ++n) u[((size_t)n * nx + i) * PS + q] = U[(n * LT + line) * NP + i];
-        p[(size_t)i * PS + q] = P[line * NP + i];
+        for (int n = 0; n < 3; ++n) u[((size_t)n * nx + i) * PS + q] = U[(n * LT + line) * NP + row_slot(i)];
+        p[(size_t)i * PS + q] = P[line * NP + row_slot(i)];
     }
-    if (!ok) atomicCAS(&sc->status, 0, PIBM_ERR_PIVOT);
 }
 template <int NX, int LT>
 __global__ void __launch_bounds__(LT * 32) k_lines(Geo g, double2 *__restrict__ u, double2 *__restrict__ p,
@@ -1048,7 +1024,7 @@ template <int NX> struct LinesCfg { static constexpr int LT = NX >= 256 ? 4 : 8;
 template <int NX>
 static size_t lines_smem(int lt) {
     const int np = lt == 4 ? lines_pitch<NX, 4>() : lines_pitch<NX, 8>();
-    return (size_t)(NX + 5 * lt * np + 32) * sizeof(double2) + NX * sizeof(double) + line_tw_bytes<NX / 32>();
+    return (size_t)(5 * lt * np) * sizeof(double2);
 }
 // Tensor maps of the persistent x-line kernel (lines_pipe.cuh): a field of
 // ncomp components [comp][i][PS complex] as FLOAT64 {2 PS, nx, ncomp}, box

@@ -3,102 +3,168 @@
 // Every cyclic system of velstep has constant coefficients (a = c, b on every
 // row, periodic coupling), i.e. it is a symmetric circulant matrix; the
 // reference solves it with Thomas + Sherman-Morrison (tridiagonal.F90:90-150,
-// usteptime.F90:344-349,457-468).  Here one warp solves one line exactly
-// through its eigen-decomposition; the (ky,kz) = (0,0) pressure line is not
-// circulant and keeps the reference's Thomas recursion.  Both matrices are
-// symmetric, so the same solves serve the adjoint step.
+// usteptime.F90:344-349,457-468).  With rho the root of a rho^2 + b rho + a = 0
+// inside the unit circle and S the shift x(i) -> x(i-1),
+//     a S^-1 + b + a S = c (1 - rho S)(1 - rho S^-1),   c = -a/rho,
+// so the exact solution is one forward recurrence y(i) = r(i)/c + rho y(i-1)
+// and one backward recurrence x(i) = y(i) + rho x(i+1), both cyclic.  A warp
+// holds a line as 32 blocks of R consecutive planes: each lane runs its block,
+// the block ends combine by cyclic doubling (after k steps a lane holds the
+// sum over 2^k blocks), and 1/(1 - rho^N) closes the period.  Doubling stops
+// where rho^(R 2^k) is below the last bit of anything it could be added to:
+// about one step for the viscous systems and three for most pressure lines.
+//
+// Against the eigen-decomposition by warp FFTs used before (10 butterfly
+// stages over all R elements of a lane, 4 shuffles each): two shuffles per
+// double and step for one element per lane, and 4 R + 10 multiply-adds per
+// component instead of about 30 R.  The x-line kernel went from 24 / 45 / 74 /
+// 142 / 1860 to 16 / 27 / 56 / 103 / 1209 us at 32 / 64 / 96 / 128 / 256^3 (the two
+// small ones mostly by the (0,0) line below).  Both matrices are symmetric, so
+// the same solves serve the adjoint step.
+//
+// The (ky,kz) = (0,0) pressure line is not circulant (nx-1 unknowns, zero at
+// either end, b = -2a: poisson.F90:127-142, 309-325) and is solved through its
+// Green's function, two prefix sums (dirichlet_solve); the reference's Thomas
+// recursion is a serial chain of two divisions per plane that one lane walked
+// twice per step while the GPU waited: at 64^3 it was half of the kernel.
 #pragma once
 #include "step_common.cuh"
 
 namespace pibm {
 
-// Per-lane constants of circulant_solve<R>, laid out [r][lane] so that a warp
-// reads 32 consecutive entries (the table lookups they replace stride by
-// R*bitrev(lane) and by r*lane, which alias shared-memory banks):
-//   cs[r*32 + l]       = cos(2 pi m/N), m = r + R*bitrev(l)   (eigenvalue of mode m)
-//   tr[(r-1)*32 + l]   = e^{-2 pi i (l r mod N)/N}, r = 1..R-1  (inter-stage twiddle)
-// The entries are copies of the twiddle table's, so the solve's arithmetic is
-// unchanged.
-template <int R> struct LineTw {
-    Tw tw;
-    const double *cs;
-    const double2 *tr;
-};
-template <int R> __host__ __device__ constexpr size_t line_tw_bytes() {
-    return (size_t)R * 32 * sizeof(double) + (size_t)(R - 1) * 32 * sizeof(double2);
-}
-// Fill cs and tr from the global twiddle table t (e^{-2 pi i m/N}, m < N); block-wide, caller syncs.
-template <int R> __device__ __forceinline__ void fill_line_tw(double *cs, double2 *tr, const double2 *t) {
-    constexpr int N = R * 32;
-    for (int e = threadIdx.x; e < R * 32; e += blockDim.x) {
-        const int r = e / 32, l = e % 32;
-        cs[e] = t[r + R * bitrev<32>(l)].x;
-        if (r > 0) tr[e - 32] = t[(l * r) % N];
-    }
-}
+// Slot of plane i in a line's row: a gap after every 8 planes, so that the 8
+// lanes of a shared-memory phase hit distinct 16-byte slots both when they
+// walk consecutive planes (i = lane + 32 r) and when they hold consecutive
+// blocks (i = R lane + r, R = 1, 2, 4, 8; two of the 8 share a slot for R = 3).
+__host__ __device__ __forceinline__ constexpr int row_slot(int i) { return i + (i >> 3); }
 
-// The solve on values held in registers: on entry v[r] = x[lane + 32 r], on
-// exit the solution at the same places.
-template <int R>
-__device__ __forceinline__ void circulant_solve_reg(double2 (&v)[R], double a, double b, const LineTw<R> &lt, int lane) {
-    constexpr int N = R * 32;
-    const Tw &tw = lt.tw;
-    // forward transform: group_fft<R, 32> with sign -1, its twiddles from the per-lane table
-    dft_inlane<R>(v, -1.0, tw);
+__device__ __forceinline__ double2 shfl2(double2 v, int src) {
+    return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+__device__ __forceinline__ double2 fma2(double a, double2 x, double2 y) { return make_double2(__fma_rn(a, x.x, y.x), __fma_rn(a, x.y, y.y)); }
+
+// Factors of one line's circulant system: rho, 1/c and rho^k (k <= R), and the
+// closures of the forward and backward recurrences.
+template <int R> struct Circ {
+    double rho, rc, pw[R], invf, invb, hf, hb;
+};
+// a x(i-1) + b x(i) + a x(i+1), b^2 > 4 a^2.  hw: x(i + N) = x(i)/hw (1 for the
+// periodic systems; the scalar's lines carry the heat ratio): the forward
+// recurrence picks up hw across the period, the backward one 1/hw.
+template <int R, bool kTwist = false>
+__device__ __forceinline__ Circ<R> circ_factor(double a, double b, double hw = 1.0) {
+    Circ<R> k;
+    const double s = __dsqrt_rn(__dmul_rn(__dsub_rn(b, __dmul_rn(2.0, a)), __dadd_rn(b, __dmul_rn(2.0, a))));
+    const double c = __dmul_rn(0.5, __dadd_rn(b, copysign(s, b)));
+    k.rc = 1.0 / c;
+    k.rho = -(a / c);
+    k.pw[0] = k.rho;
 #pragma unroll
-    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], lt.tr[(r - 1) * 32 + lane]);
-    // Each butterfly stage in one form for both lanes of a pair (no select of
-    // two computed branches): the upper lane forms v + pv, the lower (pv - v) w,
-    // i.e. t = pv + sgn v, then t times w' with w' = 1 on the upper lane.  The
-    // last stage's twiddle is 1 on every lane: no multiply.
+    for (int r = 1; r < R; ++r) k.pw[r] = __dmul_rn(k.pw[r - 1], k.rho);
+    double pn = k.pw[R - 1];
 #pragma unroll
-    for (int h = 16; h >= 1; h >>= 1) {
-        const bool upper = (lane & h) == 0;
-        const double sgn = upper ? 1.0 : -1.0;
-        const double2 w = (upper || h == 1) ? make_double2(1.0, 0.0) : tw.stage(h, lane & (h - 1), -1.0);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const double2 pv = shfl_xor2(v[r], h, 32);
-            const double2 t = make_double2(__fma_rn(sgn, v[r].x, pv.x), __fma_rn(sgn, v[r].y, pv.y));
-            v[r] = h == 1 ? t : cmul(t, w);
-        }
+    for (int h = 1; h < 32; h <<= 1) pn = __dmul_rn(pn, pn);
+    k.hf = kTwist ? hw : 1.0;
+    k.hb = kTwist ? 1.0 / hw : 1.0;
+    k.invf = 1.0 / __dsub_rn(1.0, __dmul_rn(pn, k.hf));
+    k.invb = kTwist ? 1.0 / __dsub_rn(1.0, __dmul_rn(pn, k.hb)) : k.invf;
+    return k;
+}
+// Cyclic sum over the lanes' block ends: P(lane) = sum_j q^j P(lane -+ j), the
+// period closed by inv; a value that crosses the period's end takes factor hw.
+template <bool kBack, bool kTwist>
+__device__ __forceinline__ double2 circ_carry(double2 P, double q, double inv, double hw, int lane) {
+#pragma unroll 1
+    for (int h = 1; h < 32 && fabs(q) > 1e-22; h <<= 1) {   // q is the line's: one branch per warp
+        const int src = kBack ? lane + h : lane - h;
+        const double2 t = shfl2(P, src & 31);
+        P = fma2(kTwist && (src & ~31) ? __dmul_rn(q, hw) : q, t, P);
+        q = __dmul_rn(q, q);
     }
-    // lane holds modes m = r + R*bitrev(lane)
+    const int src = kBack ? lane + 1 : lane - 1;
+    double2 y = shfl2(P, src & 31);
+    const double f = kTwist && (src & ~31) ? __dmul_rn(inv, hw) : inv;
+    return make_double2(__dmul_rn(f, y.x), __dmul_rn(f, y.y));
+}
+// The solve on a lane's block: on entry v[r] = right-hand side at plane
+// R lane + r, on exit the solution there.
+template <int R, bool kTwist = false>
+__device__ __forceinline__ void circ_solve(double2 (&v)[R], const Circ<R> &k, int lane) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const double lam = ((double)N) * (b + 2.0 * a * lt.cs[r * 32 + lane]), rlam = 1.0 / lam;
-        v[r] = make_double2(qdiv(v[r].x, lam, rlam), qdiv(v[r].y, lam, rlam));
+        v[r] = make_double2(__dmul_rn(v[r].x, k.rc), __dmul_rn(v[r].y, k.rc));
+        if (r > 0) v[r] = fma2(k.rho, v[r - 1], v[r]);
     }
-    // exact inverse of the forward stages (unnormalised; 1/N folded into lam)
-    // Inverse stages: the lower lane of a pair first multiplies its own value by
-    // conj w (the upper by 1), then both take pv + sgn v: upper u + l conj w,
-    // lower u - l conj w.
+    double2 y = circ_carry<false, kTwist>(v[R - 1], k.pw[R - 1], k.invf, k.hf, lane);
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = fma2(k.pw[r], y, v[r]);
+#pragma unroll
+    for (int r = R - 2; r >= 0; --r) v[r] = fma2(k.rho, v[r + 1], v[r]);
+    y = circ_carry<true, kTwist>(v[0], k.pw[R - 1], k.invb, k.hb, lane);
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = fma2(k.pw[R - 1 - r], y, v[r]);
+}
+// The (0,0) pressure line: a (x(i-1) - 2 x(i) + x(i+1)) = r(i) for planes
+// 0..N-2 with x(-1) = x(N-1) = 0, on the real parts; x(N-1) = 0 and the
+// imaginary parts 0.  With f = r/a,
+//   x(i) = -( (N-1-i) sum_{k<=i} (k+1) f(k) + (i+1) sum_{k>i} (N-1-k) f(k) )/N.
+template <int R>
+__device__ __forceinline__ void dirichlet_solve(double2 (&v)[R], double a, int lane) {
+    constexpr int N = 32 * R;
+    const int i0 = R * lane;
+    double A[R], B[R];   // inclusive prefix of (k+1) f, exclusive suffix of (N-1-k) f within the block
+    double sa = 0.0, sb = 0.0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const double f = i0 + r < N - 1 ? v[r].x / a : 0.0;
+        sa = __fma_rn((double)(i0 + r + 1), f, sa);
+        A[r] = sa;
+        B[r] = __dmul_rn((double)(N - 1 - i0 - r), f);
+    }
+#pragma unroll
+    for (int r = R - 1; r >= 0; --r) {
+        const double t = B[r];
+        B[r] = sb;
+        sb = __dadd_rn(sb, t);
+    }
+    double pa = sa, pb = sb;
 #pragma unroll
     for (int h = 1; h < 32; h <<= 1) {
-        const bool upper = (lane & h) == 0;
-        const double sgn = upper ? 1.0 : -1.0;
-        const double2 w = (upper || h == 1) ? make_double2(1.0, 0.0) : tw.stage(h, lane & (h - 1), +1.0);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const double2 m = h == 1 ? v[r] : cmul(v[r], w);
-            const double2 pv = shfl_xor2(m, h, 32);
-            v[r] = make_double2(__fma_rn(sgn, m.x, pv.x), __fma_rn(sgn, m.y, pv.y));
-        }
+        const double ta = __shfl_up_sync(0xffffffffu, pa, h), tb = __shfl_down_sync(0xffffffffu, pb, h);
+        if (lane >= h) pa = __dadd_rn(pa, ta);
+        if (lane + h < 32) pb = __dadd_rn(pb, tb);
     }
+    pa = __shfl_up_sync(0xffffffffu, pa, 1);
+    pb = __shfl_down_sync(0xffffffffu, pb, 1);
+    if (lane == 0) pa = 0.0;
+    if (lane == 31) pb = 0.0;
 #pragma unroll
-    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], cconj(lt.tr[(r - 1) * 32 + lane]));
-    dft_inlane<R>(v, +1.0, tw);
+    for (int r = 0; r < R; ++r) {
+        const int i = i0 + r;
+        const double t = __fma_rn((double)(N - 1 - i), __dadd_rn(A[r], pa), __dmul_rn((double)(i + 1), __dadd_rn(B[r], pb)));
+        v[r] = make_double2(i < N - 1 ? -(t / (double)N) : 0.0, 0.0);
+    }
 }
-// The solve on row[0..N-1] in shared memory (one warp, in place).
-template <int R>
-__device__ __forceinline__ void circulant_solve(double2 *row, double a, double b, const LineTw<R> &lt, int lane) {
+// Solve on a row in shared memory (plane i at row[row_slot(i)]; one warp, in
+// place): the (0,0) line's Dirichlet problem or the circulant one.
+template <int R, bool kTwist = false>
+__device__ __forceinline__ void circ_solve_row(double2 *row, const Circ<R> &k, int lane) {
     double2 v[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = row[lane + 32 * r];
-    circulant_solve_reg<R>(v, a, b, lt, lane);
-    __syncwarp();
+    for (int r = 0; r < R; ++r) v[r] = row[row_slot(R * lane + r)];
+    circ_solve<R, kTwist>(v, k, lane);
 #pragma unroll
-    for (int r = 0; r < R; ++r) row[lane + 32 * r] = v[r];
+    for (int r = 0; r < R; ++r) row[row_slot(R * lane + r)] = v[r];
+    __syncwarp();
+}
+template <int R>
+__device__ __forceinline__ void dirichlet_solve_row(double2 *row, double a, int lane) {
+    double2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = row[row_slot(R * lane + r)];
+    dirichlet_solve<R>(v, a, lane);
+#pragma unroll
+    for (int r = 0; r < R; ++r) row[row_slot(R * lane + r)] = v[r];
     __syncwarp();
 }
 
@@ -212,25 +278,6 @@ __device__ __forceinline__ void divcorr_update(const LineCoef &k, double2 d0, do
     const double2 lap = make_double2(__dsub_rn(qdiv(__dadd_rn(__dsub_rn(dm.x, __dmul_rn(2.0, d0.x)), dp.x), dx2, rdx2), __dmul_rn(w2, d0.x)),
                                      __dsub_rn(qdiv(__dadd_rn(__dsub_rn(dm.y, __dmul_rn(2.0, d0.y)), dp.y), dx2, rdx2), __dmul_rn(w2, d0.y)));
     np = make_double2(__dsub_rn(__dadd_rn(Pw.x, d0.x), __dmul_rn(k.c2dtv, lap.x)), __dsub_rn(__dadd_rn(Pw.y, d0.y), __dmul_rn(k.c2dtv, lap.y)));
-}
-
-// Thomas recursion (tridag, tridiagonal.F90:47-87) on the real parts of
-// row[0..n-1]; constant a, b, c; result in row[].x, row[].y = 0, row[n] = 0.
-__device__ __forceinline__ bool thomas_real(double2 *row, double *gam, double a, double b, double c, int n) {
-    double bet = b;
-    if (bet == 0.0) return false;
-    double prev = row[0].x / bet;
-    row[0] = make_double2(prev, 0.0);
-    for (int j = 1; j < n; ++j) {
-        gam[j] = c / bet;
-        bet = b - a * gam[j];
-        if (bet == 0.0) return false;
-        prev = (row[j].x - a * prev) / bet;
-        row[j] = make_double2(prev, 0.0);
-    }
-    for (int j = n - 2; j >= 0; --j) row[j].x = row[j].x - gam[j + 1] * row[j + 1].x;
-    row[n] = make_double2(0.0, 0.0);
-    return true;
 }
 
 }  // namespace pibm

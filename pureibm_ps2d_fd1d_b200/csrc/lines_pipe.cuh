@@ -47,13 +47,9 @@ template <int NX> struct LPipe {
     static constexpr int O_RING = 0;
     static constexpr int O_P = O_RING + KR * SLAB;           // p tile (TMA store source)
     static constexpr int O_U = O_P + SLAB;                   // 3 u tiles (TMA store sources)
-    static constexpr int O_ROW = O_U + 3 * SLAB;             // per-warp rows [LT][NX] double2
-    static constexpr int O_TWS = O_ROW + LT * NX * 16;       // twiddles, NX double2
-    static constexpr int O_ST = O_TWS + NX * 16;             // stage table, 32 double2
-    static constexpr int O_LCS = O_ST + 32 * 16;             // per-lane cosines, R*32 doubles
-    static constexpr int O_LTR = O_LCS + R * 32 * 8;         // per-lane twiddles, (R-1)*32 double2
-    static constexpr int O_GAM = O_LTR + (R - 1) * 32 * 16;  // Thomas scratch, NX doubles
-    static constexpr int O_BAR = O_GAM + NX * 8;             // full[KR], empty[KR]
+    static constexpr int NXP = NX + NX / 8;                  // a line's padded row (row_slot)
+    static constexpr int O_ROW = O_U + 3 * SLAB;             // per-warp rows [LT][NXP] double2
+    static constexpr int O_BAR = O_ROW + LT * NXP * 16;      // full[KR], empty[KR]
     static constexpr int O_TID = O_BAR + 2 * KR * 8;         // ticket of the tile in flight, 2 ints
     static constexpr int BYTES = O_TID + 16;
     static constexpr int SMEM = BYTES + 1024;                // + alignment slack
@@ -80,11 +76,6 @@ __device__ __forceinline__ void lines_pipe_body(const Geo &g, const LineMaps &mp
     extern __shared__ unsigned char lp_raw[];
     unsigned char *sm = lp_raw + ((1024u - (smem_u32(lp_raw) & 1023u)) & 1023u);
     unsigned char *ring = sm + L::O_RING, *Pt = sm + L::O_P, *Ut = sm + L::O_U;   // u tile n at Ut + n*SLAB
-    double2 *tws = reinterpret_cast<double2 *>(sm + L::O_TWS);
-    double2 *st = reinterpret_cast<double2 *>(sm + L::O_ST);
-    double *lcs = reinterpret_cast<double *>(sm + L::O_LCS);
-    double2 *ltr = reinterpret_cast<double2 *>(sm + L::O_LTR);
-    double *gam = reinterpret_cast<double *>(sm + L::O_GAM);
     uint64_t *full = reinterpret_cast<uint64_t *>(sm + L::O_BAR), *empty = full + KR;
     volatile int *tid_ring = reinterpret_cast<int *>(sm + L::O_TID);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -92,11 +83,8 @@ __device__ __forceinline__ void lines_pipe_body(const Geo &g, const LineMaps &mp
 
     if (threadIdx.x == 0)
         for (int k = 0; k < KR; ++k) { mbar_init(full + k, 1); mbar_init(empty + k, L::LT); }
-    for (int t = threadIdx.x; t < NX; t += blockDim.x) tws[t] = g.tw[t];
-    fill_stage_table<32>(st, g.tw, NX);
-    fill_line_tw<R>(lcs, ltr, g.tw);
-    grid_dep_wait();   // the tables above are set-up data; the fields and the status come from earlier kernels
-    // one barrier: the early-return vote, the barrier inits and the tables
+    grid_dep_wait();   // the fields and the status come from earlier kernels
+    // one barrier: the early-return vote and the barrier inits
     const bool failed = block_failed(sc);
 
     if (!failed && warp == L::LT) {
@@ -123,12 +111,10 @@ __device__ __forceinline__ void lines_pipe_body(const Geo &g, const LineMaps &mp
     } else if (!failed) {
         // ---------------- consumers: warp w solves line 4 t + w ----------------
         const int w = warp;
-        const LineTw<R> tw{{tws, NX, 1, st}, lcs, ltr};
         const double dx = g.dx, dx2 = g.dx2, dt = sc->dt, vis = g.vis;
         const double c1 = g.c1, c2 = g.c2, c3 = g.c3, c4 = g.c4;
         const double c12 = c1 + c2, rdx = 1.0 / dx, rdx2 = 1.0 / dx2, rc12 = 1.0 / c12;
-        double2 *row = reinterpret_cast<double2 *>(sm + L::O_ROW) + w * NX;   // this warp's scratch row
-        bool ok = true;
+        double2 *row = reinterpret_cast<double2 *>(sm + L::O_ROW) + w * L::NXP;   // this warp's scratch row
         uint32_t k = 0;
         auto next_slab = [&](bool wait_done) -> unsigned char * {
             const int slot = k % KR;
@@ -139,6 +125,13 @@ __device__ __forceinline__ void lines_pipe_body(const Geo &g, const LineMaps &mp
             __syncwarp();
             if (lane == 0) mbar_arrive(empty + (k % KR));
             ++k;
+        };
+        // the solve of strided values v[r] = x[lane + 32 r]: through the row into blocks of R planes
+        auto to_row = [&](const double2 (&v)[R]) {
+            __syncwarp();   // every lane is done with the row's last contents
+#pragma unroll
+            for (int r = 0; r < R; ++r) row[row_slot(lane + 32 * r)] = v[r];
+            __syncwarp();
         };
         for (int c = 0;; ++c) {
             if (!mbar_wait(full + (k % KR), (k / KR) & 1)) atomicCAS(&sc->status, 0, PIBM_ERR_TIMEOUT);
@@ -182,21 +175,15 @@ __device__ __forceinline__ void lines_pipe_body(const Geo &g, const LineMaps &mp
             }
 #pragma unroll
             for (int r = 0; r < R; ++r) v[r] = make_double2(qdiv(tt[r].x, c12, rc12), qdiv(tt[r].y, c12, rc12));
-            if (q == 0) {
+            const Circ<R> kp = circ_factor<R>(kw.pa, kw.pb);
+            to_row(v);
+            if (q == 0) dirichlet_solve_row<R>(row, kw.pa, lane);
+            else circ_solve_row<R>(row, kp, lane);
 #pragma unroll
-                for (int r = 0; r < R; ++r) row[lane + 32 * r] = v[r];
-                __syncwarp();
-                if (lane == 0) ok = thomas_real(row, gam, kw.pa, kw.pb, kw.pc, NX - 1) && ok;
-                __syncwarp();
-#pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = row[lane + 32 * r];
-            } else {
-                circulant_solve_reg<R>(v, kw.pa, kw.pb, tw, lane);
-            }
-#pragma unroll
-            for (int r = 0; r < R; ++r) tel(Pt, lane + 32 * r, w) = p_update(po[r], v[r]);
+            for (int r = 0; r < R; ++r) tel(Pt, lane + 32 * r, w) = p_update(po[r], row[row_slot(lane + 32 * r)]);
             __syncwarp();
             // ---- ustep per component (usteptime.F90:73-470)
+            const Circ<R> ku = circ_factor<R>(kw.ua, kw.ub);
 #pragma unroll 1
             for (int n = 0; n < 3; ++n) {
                 unsigned char *S = next_slab(false);
@@ -209,9 +196,10 @@ __device__ __forceinline__ void lines_pipe_body(const Geo &g, const LineMaps &mp
                                       kz, dx, rdx, dx2, rdx2);
                 }
                 release();
-                circulant_solve_reg<R>(rr, kw.ua, kw.ub, tw, lane);
+                to_row(rr);
+                circ_solve_row<R>(row, ku, lane);
 #pragma unroll
-                for (int r = 0; r < R; ++r) tel(U, lane + 32 * r, w) = rr[r];
+                for (int r = 0; r < R; ++r) tel(U, lane + 32 * r, w) = row[row_slot(lane + 32 * r)];
             }
             __syncwarp();
             unsigned char *U1 = Ut, *U2 = Ut + L::SLAB, *U3 = Ut + 2 * L::SLAB;
@@ -224,25 +212,16 @@ __device__ __forceinline__ void lines_pipe_body(const Geo &g, const LineMaps &mp
                                             dx, rdx);
                 v[r] = make_double2(qdiv(t2.x, kw.alp, ralpc), qdiv(t2.y, kw.alp, ralpc));
             }
-            if (q == 0) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) row[lane + 32 * r] = v[r];
-                __syncwarp();
-                if (lane == 0) ok = thomas_real(row, gam, kw.pa, kw.pb, kw.pc, NX - 1) && ok;
-                __syncwarp();
-            } else {
-                circulant_solve_reg<R>(v, kw.pa, kw.pb, tw, lane);
-#pragma unroll
-                for (int r = 0; r < R; ++r) row[lane + 32 * r] = v[r];
-                __syncwarp();
-            }
+            to_row(v);
+            if (q == 0) dirichlet_solve_row<R>(row, kw.pa, lane);
+            else circ_solve_row<R>(row, kp, lane);
             {
                 double2 nu1[R], nu2[R], nu3[R], np[R];
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const int i = lane + 32 * r;
                     const int im = i == 0 ? NX - 1 : i - 1, ip = i == NX - 1 ? 0 : i + 1;
-                    divcorr_update(kw, row[i], row[im], row[ip], i == 0, tel(U1, i, w), tel(U2, i, w), tel(U3, i, w), tel(Pt, i, w), ky, kz, w2w,
+                    divcorr_update(kw, row[row_slot(i)], row[row_slot(im)], row[row_slot(ip)], i == 0, tel(U1, i, w), tel(U2, i, w), tel(U3, i, w), tel(Pt, i, w), ky, kz, w2w,
                                    dx, rdx, dx2, rdx2, nu1[r], nu2[r], nu3[r], np[r]);
                 }
                 __syncwarp();
@@ -273,7 +252,6 @@ __device__ __forceinline__ void lines_pipe_body(const Geo &g, const LineMaps &mp
                 bulk_commit();
             }
         }
-        if (!ok) atomicCAS(&sc->status, 0, PIBM_ERR_PIVOT);
         if (threadIdx.x == 0) bulk_wait_all();
     }
     // the last block to finish resets the tickets for the next launch

@@ -24,6 +24,7 @@
 //            corners                                      [phistep]
 //   k_sfin   heat_ratio update, Nusselt number, status
 #include "step_common.cuh"
+#include "line_solve.cuh"
 
 namespace pibm {
 
@@ -552,82 +553,20 @@ __global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) k_sff(Geo g, const doub
 // k_slines: phistep per (ky,kz) line (stepthescalar.F90:99-213).  The system
 //   a x(i-1) + b x(i) + c x(i+1) = r(i),  x(0) = H x(nx),  x(nx+1) = x(1)/H,
 // H = heat_ratio_new, a = c (the reference's tridag3 + Sherman-Morrison with
-// corners a*H and c/H) becomes circulant under x(i) = mu^i y(i), mu^nx = 1/H:
-//   (a/mu) y(i-1) + b y(i) + (a mu) y(i+1) = r(i) mu^-i,  y periodic,
-// and one warp solves it exactly through its eigenvalues
-//   lambda_m = b + a (mu + 1/mu) cos(2 pi m/nx) + i a (mu - 1/mu) sin(2 pi m/nx)
-// with a forward FFT in registers, a complex division and the exact inverse.
-// LT lines per CTA; loads run over consecutive lines (coalesced).
+// corners a*H and c/H), is the circulant solve of the flow's x lines with a
+// solution that is periodic up to the factor H (circ_solve, kTwist): one warp
+// per line, LT lines per CTA; loads run over consecutive lines (coalesced).
 // ============================================================================
-template <int R>
-__device__ __forceinline__ void twisted_solve(double2 *row, double a, double b, double mpl, double mmi,
-                                              const double *pw, const double *ipw, const Tw &tw, int lane) {
-    constexpr int N = R * 32;
-    double2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int i = lane + 32 * r;
-        const double2 x = row[i];
-        v[r] = make_double2(x.x * ipw[i], x.y * ipw[i]);
-    }
-    group_fft<R, 32>(v, lane, -1.0, tw);
-    const int br = bitrev<32>(lane);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int m = r + R * br;
-        const double2 e = tw.t[m * tw.stride];   // (cos, -sin)
-        const double lr = (double)N * (b + a * mpl * e.x), li = (double)N * (a * mmi * (-e.y));
-        const double den = lr * lr + li * li, rden = 1.0 / den;
-        v[r] = make_double2(qdiv(v[r].x * lr + v[r].y * li, den, rden), qdiv(v[r].y * lr - v[r].x * li, den, rden));
-    }
-    // inverse stages: the lower lane of a pair first multiplies its own value
-    // by conj w (the upper by 1), then both take pv + sgn v
-#pragma unroll
-    for (int h = 1; h < 32; h <<= 1) {
-        const bool upper = (lane & h) == 0;
-        const double sgn = upper ? 1.0 : -1.0;
-        const double2 w = (upper || h == 1) ? make_double2(1.0, 0.0) : tw.stage(h, lane & (h - 1), +1.0);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const double2 m = h == 1 ? v[r] : cmul(v[r], w);   // the first stage's twiddle is 1
-            const double2 pv = shfl_xor2(m, h, 32);
-            v[r] = make_double2(__fma_rn(sgn, m.x, pv.x), __fma_rn(sgn, m.y, pv.y));
-        }
-    }
-#pragma unroll
-    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw.get((lane * r) % N, +1.0));
-    dft_inlane<R>(v, +1.0, tw);
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int i = lane + 32 * r;
-        row[i] = make_double2(v[r].x * pw[i], v[r].y * pw[i]);
-    }
-    __syncwarp();
-}
-
 template <int NX, int LT>
 __global__ void __launch_bounds__(LT * 32) k_slines(Geo g, double2 *__restrict__ phif, const double2 *__restrict__ nln,
                                                     const double2 *__restrict__ nlo, const double2 *__restrict__ ffs,
                                                     Scal *__restrict__ sc) {
     constexpr int R = NX / 32, NP = lines_pitch<NX, LT>();
     extern __shared__ double2 sm[];
-    double2 *tws = sm;
-    double2 *RHS = tws + NX;                       // [line][i], pitch NP
-    double *pw = (double *)(RHS + LT * NP);        // mu^(i+1)
-    double *ipw = pw + NX;                         // mu^-(i+1)
-    double2 *st = (double2 *)(ipw + NX);           // cross-lane stage twiddles
+    double2 *RHS = sm;                             // [line][i], pitch NP
     if (block_failed(sc)) return;
-    fill_stage_table<32>(st, g.tw, NX);
     const int PS = g.PS, nx = NX;
     const double h = sc->heat_ratio, H = sc->heat_ratio_new;
-    for (int t = threadIdx.x; t < NX; t += blockDim.x) {
-        tws[t] = g.tw[t];
-        const double lg = log(H) / (double)NX;
-        pw[t] = exp(-(double)(t + 1) * lg);
-        ipw[t] = exp((double)(t + 1) * lg);
-    }
-    const double mu = exp(-log(H) / (double)NX), imu = 1.0 / mu;
     const int q0 = blockIdx.x * LT;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const double dt = sc->dt, gm = g.gamma_s, dx2 = g.dx2, rdx2 = 1.0 / dx2;
@@ -656,28 +595,27 @@ __global__ void __launch_bounds__(LT * 32) k_slines(Geo g, double2 *__restrict__
             const double2 pp = PF(2, q), pm = PF(nx, q);
             lap = make_double2((pp.x - 2.0 * pc.x) + pm.x * h, (pp.y - 2.0 * pc.y) + pm.y * h);
         }
-        RHS[line * NP + (i - 1)] = make_double2(r.x + qdiv(k1 * lap.x, dx2, rdx2), r.y + qdiv(k1 * lap.y, dx2, rdx2));
+        RHS[line * NP + row_slot(i - 1)] = make_double2(r.x + qdiv(k1 * lap.x, dx2, rdx2), r.y + qdiv(k1 * lap.y, dx2, rdx2));
     }
     __syncthreads();
     const int qw = q0 + w;
     if (qw < PS) {
         const double a = -(dt * gm * c2 / dx2);
         const double bd = 1.0 + dt * gm * c2 * (2.0 / dx2 + g.w2[qw]);
-        const Tw tw{tws, NX, 1, st};
-        twisted_solve<R>(RHS + w * NP, a, bd, mu + imu, mu - imu, pw, ipw, tw, lane);
+        circ_solve_row<R, true>(RHS + w * NP, circ_factor<R, true>(a, bd, H), lane);
     }
     __syncthreads();
     for (int t = threadIdx.x; t < LT * NX; t += blockDim.x) {
         const int line = t % LT, i = t / LT, q = q0 + line;
         if (q >= PS) continue;
-        phif[(size_t)i * PS + q] = RHS[line * NP + i];
+        phif[(size_t)i * PS + q] = RHS[line * NP + row_slot(i)];
     }
 }
 template <int NX> struct SLinesCfg { static constexpr int LT = NX >= 256 ? 4 : 8; };
 template <int NX>
 static size_t slines_smem() {
     constexpr int LT = SLinesCfg<NX>::LT;
-    return (size_t)(NX + LT * lines_pitch<NX, LT>() + 32) * sizeof(double2) + 2 * NX * sizeof(double);
+    return (size_t)(LT * lines_pitch<NX, LT>()) * sizeof(double2);
 }
 
 // heat_ratio update, surface flux and Nusselt number (bcsetscal, bc_scalar.F90:186-190,

@@ -68,6 +68,41 @@ def test_single_sphere_32_steps(scheme, limiter):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("my,re,width", [(32, 0.05, 4), (32, 20.0, 8), (64, 0.05, 8), (64, 20.0, 4), (96, 0.05, 4), (96, 20.0, 8),
+                                         (128, 0.05, 4), (128, 0.05, 8), (256, 0.05, 4), (256, 20.0, 8)])
+def test_line_solves_of_a_rough_state(my, re, width):
+    """Two steps from a random state with every (ky,kz) line and x mode excited,
+    the (0,0) line included: at Re 0.05 (nu dt/dx^2 of order 100) the viscous
+    systems couple a whole line, at Re 20 a few planes.  Bound: the pressure
+    lines' condition number, up to (N/pi)^2 = 7e3 at 256, times a few roundings."""
+    prm, xc = config.single_sphere(my=my, dia_cells=8.0, re=re)
+    gpu, cpu = make_pair(prm, xc)
+    gpu.set_tuning(width)
+    rng, uchar = np.random.default_rng(my), re * prm["vis"]
+    st = gpu.get_state()
+    for k in ("u", "nl", "p"):
+        shp = st[k].shape
+        a = rng.standard_normal(shp) + 1j * rng.standard_normal(shp)
+        if k != "p":
+            a[..., -1] = a[..., 0]      # the periodic image plane
+        st[k] = a * (uchar / my * (0.1 if k == "u" else 0.01))
+    real = np.fft.rfft2(np.fft.irfft2(np.moveaxis(st["u"], 3, 1), s=(my, my)))   # the spectra of real fields
+    st["u"] = np.ascontiguousarray(np.moveaxis(real, 1, 3))
+    real = np.fft.rfft2(np.fft.irfft2(np.moveaxis(st["nl"], 3, 1), s=(my, my)))
+    st["nl"] = np.ascontiguousarray(np.moveaxis(real, 1, 3))
+    gpu.set_state(st)
+    cpu.set_state(st)
+    for _ in range(2):
+        gpu.step()
+        cpu.step()
+    # the solved fields; the mpg controller is cf = -1/dt times a difference of
+    # means of the random field, in which the two summation orders' last bits
+    # (2e-16 x 16 M terms) show as 5e-10
+    sg, sc = gpu.get_state(), cpu.get_state()
+    assert max(rel(sg[k], sc[k]) for k in ("u", "p", "nl")) <= TOL
+
+
+@pytest.mark.gpu
 def test_single_sphere_64_100_steps():
     """Single fixed sphere, 64^3, d=16, Re=20, fluid at rest, 100 steps."""
     prm, xc = config.single_sphere(my=64, dia_cells=16, re=20.0)
