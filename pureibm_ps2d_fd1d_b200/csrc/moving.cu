@@ -9,7 +9,9 @@
 // to a serial evaluation of the same expressions.
 //
 // The reference keeps the contact lists with one sequential loop over the
-// particles.  Here each sub-step is three launches:
+// particles.  Here all sub-steps of a flow step run in one launch of one
+// thread-block cluster (k_dem_march), up to kMarchMax particles; larger
+// systems, which need the whole GPU, take three launches per sub-step:
 //   k_dem_update  one thread per particle L: every pair (J, L) is evaluated by
 //                 both its threads with the same arithmetic; L applies what the
 //                 serial loop does to L's list at J's turn (J < L), then at
@@ -23,8 +25,11 @@
 // What makes this exact: within a sub-step the reference changes L's entries
 // for a partner P > L only at L's own turn and its entries for P < L only at
 // P's turn, so every decision reads lists as they were at the sub-step start.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "step_common.cuh"
 
@@ -33,17 +38,20 @@ namespace pibm {
 namespace {
 
 constexpr double kPiD = 3.14159265358979323846;
+// Squared distances beyond this factor of a squared radius (below its inverse)
+// are decided without the square root: far outside the roundings of either.
+constexpr double kFar = 1.0 + 1e-9;
 
 // One contact pair as CALC_FORCE_DES evaluates it at LL = A's turn, I = B
 // (soft_sphere_coll.F90:300-420, CFRELVEL :728-776): periodic unwrap of B,
 // overlap test, normal spring-dashpot force on A.  Reads the sub-step's
 // starting positions and velocities.
-__device__ bool pair_force(const Mov &m, int A, int B, double fn[3], Scal *sc) {
+__device__ __forceinline__ bool pair_force(const Mov &m, const double *pos, const double *vel, int A, int B, double fn[3], Scal *sc) {
     const double L3[3] = {m.XL, m.YL, m.ZL};
     double pB[3], dist[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const double a = m.pos_old[3 * A + d], b = m.pos_old[3 * B + d];
+        const double a = pos[3 * A + d], b = pos[3 * B + d];
         pB[d] = b;
         if (fabs(a - b) > 4.0 * m.max_radius) pB[d] = b > a ? b - L3[d] : b + L3[d];
         dist[d] = pB[d] - a;
@@ -52,6 +60,7 @@ __device__ bool pair_force(const Mov &m, int A, int B, double fn[3], Scal *sc) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) dd = dd + dist[d] * dist[d];
     const double rlm = m.rad + m.rad;
+    if (dd > rlm * rlm * kFar) return false;   // apart whatever the roundings of the test below
     const double distmod = sqrt(dd);
     if (!(rlm - distmod > kSmallD)) return false;
     if (distmod == 0.0) { atomicCAS(&sc->status, 0, PIBM_ERR_DEM_MOVE); return false; }
@@ -59,7 +68,7 @@ __device__ bool pair_force(const Mov &m, int A, int B, double fn[3], Scal *sc) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         nrm[d] = dist[d] / distmod;
-        vrel[d] = m.vel_old[3 * A + d] - m.vel_old[3 * B + d];
+        vrel[d] = vel[3 * A + d] - vel[3 * B + d];
         osum[d] = 0.0 * m.rad + 0.0 * m.rad;   // OMEGA stays zero (rotation update disabled)
     }
     const double vrot[3] = {osum[1] * nrm[2] - osum[2] * nrm[1], osum[2] * nrm[0] - osum[0] * nrm[2],
@@ -118,13 +127,13 @@ __global__ void __launch_bounds__(32 * kUpdWarps) k_dem_update(Mov m, Scal *sc, 
         int f = 0;
         double fn[3] = {0.0, 0.0, 0.0};
         if (P < L) {
-            if (pair_force(m, P, L, fn, sc)) {
+            if (pair_force(m, m.pos_old, m.vel_old, P, L, fn, sc)) {
                 f = 1;
                 for (int p = 0; p < m.pncnt[P]; ++p)
                     if (m.pn[P * MX + p] == L) { if (m.pv[P * MX + p] == 1) f |= 2; break; }
             }
         } else if (P > L) {
-            if (pair_force(m, L, P, fn, sc)) f = 1;
+            if (pair_force(m, m.pos_old, m.vel_old, L, P, fn, sc)) f = 1;
         }
         cf_s[wid][q] = f;
 #pragma unroll
@@ -432,6 +441,347 @@ __global__ void __launch_bounds__(32 * kSearchWarps) k_dem_search(Mov m, Scal *s
     const int pc = m.pncnt2[L];
     for (int q = lane; q < pc; q += 32) { m.pn[L * MX + q] = m.pn2[L * MX + q]; m.pv[L * MX + q] = m.pv2[L * MX + q]; }
     if (lane == 0) m.pncnt[L] = pc;
+}
+
+// ============================================================================
+// k_dem_march: every sub-step of one flow step (CALC_FORCE_DES, CFNEWVALUES,
+// the neighbour search and CFUPDATEOLD, as k_dem_update / k_dem_bin /
+// k_dem_search run them) in one launch: one cluster of up to 8 CTAs, a warp
+// per particle (in turn when there are more), one cluster barrier per
+// sub-step.  Every CTA keeps all positions, velocities and cells in shared
+// memory, in two buffers that ping-pong: the warp that advances a particle
+// stores them into each CTA's copy, and may search with the new positions and
+// start its next update while others still search.  Neighbour lists stay in
+// the shared memory of their particle's CTA; contact lists, which are mostly
+// empty and read by a partner only in contact, ping-pong in global memory.
+//
+// The search needs no bins: a warp keeps the particles within the search
+// radius plus a skin (kSkin radii) of its own as candidates, rebuilt from all
+// pairs when any particle has moved half the skin since (a flow step moves
+// them by a small fraction of a cell).  Each candidate is put through the
+// reference's test for every one of the 27 neighbourhood cells that its cell
+// matches, and the finds are ordered as the cell scan finds them, so the
+// lists are those of the serial loop whatever the coarse grid.
+//
+// Bound: a chain of dependent shared-memory reads and FP64 arithmetic per
+// particle, and the barrier: 1.9 us of update, 1.4 us of search and 1.7 us of
+// barrier per sub-step with 43 particles on eight SMs, 4.9 us against 16.5 us
+// for the three launches.
+// ============================================================================
+// Particles.  Eight SMs take 41 us per sub-step with 1202 (their FP64 pipes are
+// full), the three launches over the whole GPU 33; the lines cross near 700.
+constexpr int kMarchMax = 512;
+constexpr int kMarchCtas = 8;      // portable cluster size
+constexpr int kMaxCand = 48;
+constexpr double kSkin = 0.4;      // in particle radii, on top of 2.4 (the search radius)
+struct MarchWarp {
+    double fn[kMaxList][3], fc[4];
+    int wl[kMaxList], wv[kMaxList];
+    unsigned short id[kMaxList], own[kMaxList], mir[kMaxList], key[kMaxList];
+    unsigned char cf[kMaxList];
+};
+// Shared-memory layout of a CTA (the same in every CTA of the cluster).
+struct MarchMem {
+    double *P[2], *V[2], *pcand, *hyd;   // [3*l + d] of all particles; of the CTA's own: candidates' base, fluid force / mass
+    int *cell[2], *flags, *pcs;          // packed cells of all; 3 rotating flag words; contact counts held in either global buffer
+    unsigned short *nb, *cand;
+    unsigned char *nbc, *cdc;
+    MarchWarp *w;
+    __host__ __device__ static size_t bytes(int N, int slots, int maxn, int warps) {
+        return (size_t)N * (12 * 8 + 8) + (size_t)slots * (6 * 8 + 8 + (maxn + kMaxCand) * 2 + 2) + 64 + warps * sizeof(MarchWarp);
+    }
+    __device__ MarchMem(unsigned char *base, int N, int slots, int maxn, int warps) {
+        w = (MarchWarp *)base;
+        double *d = (double *)(base + warps * sizeof(MarchWarp));
+        for (int b = 0; b < 2; ++b) { P[b] = d; d += 3 * N; }
+        for (int b = 0; b < 2; ++b) { V[b] = d; d += 3 * N; }
+        pcand = d; d += 3 * slots;
+        hyd = d; d += 3 * slots;
+        int *q = (int *)d;
+        for (int b = 0; b < 2; ++b) { cell[b] = q; q += N; }
+        pcs = q; q += 2 * slots;
+        flags = q; q += 4;
+        nb = (unsigned short *)q;
+        cand = nb + (size_t)slots * maxn;
+        nbc = (unsigned char *)(cand + (size_t)slots * kMaxCand);
+        cdc = nbc + slots;
+    }
+};
+__device__ __forceinline__ int pack_cell(int i, int j, int k) { return i | (j << 10) | (k << 20); }
+__device__ __forceinline__ int cell_dir(int c, int d) { return (c >> (10 * d)) & 1023; }
+// Offset d in {-1, 0, 1} of one direction from cell c: whether it leads to
+// `target`, and the image factor through which the search sees it (nb_cell).
+__device__ __forceinline__ bool nb_dir(int c, int d, int cmax, int target, double &sh) {
+    int ii = c + d;
+    sh = 0.0;
+    if (ii > cmax) { ii = 2; sh = 1.0; }
+    if (ii < 2) { ii = cmax; sh = -1.0; }
+    return ii == target;
+}
+// First of the 27 offsets, in the reference's scan order, through which the
+// search from a particle at A (cell cA) accepts the particle at B (cell cB); 27 if none.
+__device__ __forceinline__ int first_image(const Mov &m, const double *A, int cA, const double *B, int cB) {
+    const double rlm = 1.2 * (m.rad + m.rad);
+    for (int dz = -1; dz <= 1; ++dz) {
+        double sz;
+        if (!nb_dir(cell_dir(cA, 2), dz, m.cz, cell_dir(cB, 2), sz)) continue;
+        for (int dy = -1; dy <= 1; ++dy) {
+            double sy;
+            if (!nb_dir(cell_dir(cA, 1), dy, m.cy, cell_dir(cB, 1), sy)) continue;
+            for (int dx = -1; dx <= 1; ++dx) {
+                double sx;
+                if (!nb_dir(cell_dir(cA, 0), dx, m.cx, cell_dir(cB, 0), sx)) continue;
+                const double c0 = B[0] + sx * m.LXs, c1 = B[1] + sy * m.LYs, c2 = B[2] + sz * m.LZs;
+                const double d0 = c0 - A[0], d1 = c1 - A[1], d2 = c2 - A[2];
+                double dd = 0.0;
+                dd = dd + d0 * d0;
+                dd = dd + d1 * d1;
+                dd = dd + d2 * d2;
+                if (dd > rlm * rlm * kFar) continue;
+                if (dd * kFar < rlm * rlm || rlm - sqrt(dd) > kSmallD) return (dx + 1) + 3 * (dy + 1) + 9 * (dz + 1);
+            }
+        }
+    }
+    return 27;
+}
+// Squared distance between two points of the periodic box.
+__device__ __forceinline__ double box_dist2(const Mov &m, const double *A, const double *B) {
+    const double t0 = fabs(A[0] - B[0]), t1 = fabs(A[1] - B[1]), t2 = fabs(A[2] - B[2]);
+    const double u0 = fmin(t0, fabs(m.XL - t0)), u1 = fmin(t1, fabs(m.YL - t1)), u2 = fmin(t2, fabs(m.ZL - t2));
+    return u0 * u0 + u1 * u1 + u2 * u2;
+}
+
+__global__ void __launch_bounds__(1024, 1) k_dem_march(Mov m, Scal *sc, const double *__restrict__ pres,
+                                                       const double *__restrict__ visc) {
+    extern __shared__ __align__(16) unsigned char march_s[];
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int ctas = gridDim.x, rank = blockIdx.x;
+    const int N = m.N, MX = m.maxn, slots = (N + ctas - 1) / ctas;   // particle L: CTA L % ctas, slot L / ctas
+    MarchMem S(march_s, N, slots, MX, nw);
+    MarchWarp &W = S.w[wid];
+    const bool failed = sc->status != 0;   // set by earlier kernels only: the same for every thread
+    const int F = failed ? 0 : m.factor[0];
+    const double dts = m.dts[0];
+    const int d3 = lane % 3;               // this lane's direction in CFNEWVALUES
+    const double fa = sc->frame_accln[d3], gm = (sc->mpg[d3] * m.pvol) / m.pmass;
+    const double Ld = d3 == 0 ? m.XL : d3 == 1 ? m.YL : m.ZL, dcd = d3 == 0 ? m.dxc : d3 == 1 ? m.dyc : m.dzc;
+    const double rdcd = 1.0 / dcd;
+    const int cmd = d3 == 0 ? m.cx : d3 == 1 ? m.cy : m.cz;
+    for (int q = threadIdx.x; q < 3 * N; q += blockDim.x) { S.P[0][q] = m.pos_old[q]; S.V[0][q] = m.vel_old[q]; }
+    for (int k = wid; k < slots; k += nw) {
+        const int L = k * ctas + rank;
+        if (L >= N) continue;
+        const int nc = m.ncnt[L];
+        for (int q = lane; q < nc; q += 32) S.nb[k * MX + q] = (unsigned short)m.neigh[L * MX + q];
+        if (lane < 3) {
+            const size_t q = (size_t)L + (size_t)N * lane;
+            S.hyd[3 * k + lane] = (m.rhof * (pres[q] + visc[q])) / m.pmass;
+        }
+        if (lane == 0) { S.nbc[k] = (unsigned char)nc; S.pcs[k] = m.pncnt[L]; S.pcs[slots + k] = -1; }
+    }
+    if (threadIdx.x < 3) S.flags[threadIdx.x] = 0;
+    cl.sync();
+    auto raise = [&](int f, int word) {   // in every CTA's copy of the flag word
+        for (int r = 0; r < ctas; ++r) atomicOr(cl.map_shared_rank(S.flags, r) + word, f);
+    };
+    int s = 0, c = 0;
+    for (; s < F; ++s, c ^= 1) {
+        double *const Pc = S.P[c], *const Vc = S.V[c], *const Pn = S.P[c ^ 1], *const Vn = S.V[c ^ 1];
+        int *const Cn = S.cell[c ^ 1];
+        int *const gl = c ? m.pn2 : m.pn, *const gv = c ? m.pv2 : m.pv, *const gc = c ? m.pncnt2 : m.pncnt;
+        int *const gln = c ? m.pn : m.pn2, *const gvn = c ? m.pv : m.pv2, *const gcn = c ? m.pncnt : m.pncnt2;
+        const int w3 = s % 3;
+        // ---- forces on and advance of every particle (k_dem_update) ----
+        for (int k = wid; k < slots; k += nw) {
+            const int L = k * ctas + rank;
+            if (L >= N) continue;
+            const int nc = S.nbc[k];
+            int wc = S.pcs[c * slots + k];
+            for (int q = lane; q < wc; q += 32) { W.wl[q] = __ldcg(gl + L * MX + q); W.wv[q] = __ldcg(gv + L * MX + q); }
+            bool touch = false;
+            for (int q = lane; q < nc; q += 32) {
+                const int P = S.nb[k * MX + q];
+                int f = 0;
+                double fn[3] = {0.0, 0.0, 0.0};
+                if (P < L) {
+                    if (pair_force(m, Pc, Vc, P, L, fn, sc)) {
+                        f = 1;
+                        const int np = __ldcg(gc + P);
+                        for (int p = 0; p < np; ++p)
+                            if (__ldcg(gl + P * MX + p) == L) { if (__ldcg(gv + P * MX + p) == 1) f |= 2; break; }
+                    }
+                } else if (P > L) {
+                    if (pair_force(m, Pc, Vc, L, P, fn, sc)) f = 1;
+                }
+                W.id[q] = (unsigned short)P;
+                W.cf[q] = (unsigned char)f;
+                touch = touch || f;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) W.fn[q][d] = fn[d];
+            }
+            touch = __any_sync(0xffffffffu, touch);
+            __syncwarp();
+            if (lane == 0) {
+                int *wl = W.wl, *wv = W.wv;
+                double fc[3] = {0.0, 0.0, 0.0};
+                bool over = false;
+                if (touch)
+                    for (int q = 0; q < nc; ++q) {
+                        const int J = W.id[q];
+                        if (J >= L || !(W.cf[q] & 1)) continue;
+                        if (W.cf[q] & 2) {
+                            for (int p = 0; p < wc; ++p) if (wl[p] == J) { wv[p] = 1; break; }
+                        } else if (wc + 1 < MX) {
+                            wl[wc] = J; wv[wc] = 1; ++wc;
+                        } else {
+                            over = true;
+                        }
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) fc[d] = fc[d] - W.fn[q][d];
+                    }
+                int w = 0;
+                for (int p = 0; p < wc; ++p) if (wv[p]) { wl[w] = wl[p]; ++w; }
+                wc = w;
+                for (int p = 0; p < wc; ++p) wv[p] = 0;
+                if (touch)
+                    for (int q = 0; q < nc; ++q) {
+                        const int I = W.id[q];
+                        if (I <= L || !(W.cf[q] & 1)) continue;
+                        int found = -1;
+                        for (int p = 0; p < wc; ++p) if (wl[p] == I) { found = p; break; }
+                        if (found >= 0) {
+                            wv[found] = 1;
+                        } else if (wc + 1 < MX) {
+                            wl[wc] = I; wv[wc] = 1; ++wc;
+                        } else {
+                            over = true;
+                        }
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) fc[d] = fc[d] + W.fn[q][d];
+                    }
+                if (over) { atomicCAS(&sc->status, 0, PIBM_ERR_NEIGH_OVERFLOW); raise(2, w3); }
+#pragma unroll
+                for (int d = 0; d < 3; ++d) W.fc[d] = fc[d];
+            }
+            wc = __shfl_sync(0xffffffffu, wc, 0);
+            __syncwarp();
+            if (wc > 0 || S.pcs[(c ^ 1) * slots + k] != 0) {   // else the global buffer holds the empty list already
+                for (int q = lane; q < wc; q += 32) { gln[L * MX + q] = W.wl[q]; gvn[L * MX + q] = W.wv[q]; }
+                if (lane == 0) gcn[L] = wc;
+            }
+            // CFNEWVALUES (collision_mod.F90:1335-1462), softsphere coupled to the flow: every lane its direction
+            const double fcd = W.fc[d3];
+            double a = (fcd == 0.0 ? fcd : fcd / m.pmass) + S.hyd[3 * k + d3];
+            a = a - fa;
+            a = a - gm;
+            const double po = Pc[3 * L + d3];
+            const double v = Vc[3 * L + d3] + a * dts;
+            double pn = po + v * dts;
+            const double t = pn - po;
+            double dd = 0.0;
+#pragma unroll
+            for (int e = 0; e < 3; ++e) { const double te = __shfl_sync(0xffffffffu, t, e); dd = dd + te * te; }
+            if (pn > Ld) pn = pn - (Ld - 0.0);
+            else if (pn < 0.0) pn = pn + (Ld - 0.0);
+            // FIND_CELL_INDEX (:743-762); the division only near a cell boundary
+            const double cq = pn * rdcd;
+            const int cn = (int)cq;
+            const int ci = min((cq - (double)cn > 1e-9 && (double)cn + 1.0 - cq > 1e-9 ? cn : (int)(pn / dcd)) + 2, cmd);
+            const int cell = pack_cell(__shfl_sync(0xffffffffu, ci, 0), __shfl_sync(0xffffffffu, ci, 1), __shfl_sync(0xffffffffu, ci, 2));
+            double A[3];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) A[e] = __shfl_sync(0xffffffffu, pn, e);
+            if (lane < 3 * ctas) {   // lane 3 r + d: direction d into CTA r's copy
+                const int r = lane / 3;
+                cl.map_shared_rank(Pn, r)[3 * L + d3] = pn;
+                cl.map_shared_rank(Vn, r)[3 * L + d3] = v;
+                if (d3 == 0) cl.map_shared_rank(Cn, r)[L] = cell;
+            }
+            if (lane == 0) {
+                S.pcs[(c ^ 1) * slots + k] = wc;
+                int fl = 0;
+                if (dd * kFar >= m.rad * m.rad && sqrt(dd) >= m.rad) { atomicCAS(&sc->status, 0, PIBM_ERR_DEM_MOVE); fl |= 2; }
+                if (s > 0 && !(box_dist2(m, A, S.pcand + 3 * k) < (0.49 * kSkin * m.rad) * (0.49 * kSkin * m.rad))) fl |= 1;
+                if (fl) raise(fl, w3);
+            }
+            __syncwarp();
+        }
+        cl.sync();
+        const int flags = *(volatile int *)(S.flags + w3);   // complete: set before the barrier
+        if (threadIdx.x == 0) S.flags[(s + 2) % 3] = 0;       // last read before this barrier, next set after the next one
+        if (flags & 2) { ++s; c ^= 1; break; }
+        // ---- GRID_BASED_NEIGHBOR_SEARCH at the new positions (k_dem_search) ----
+        for (int k = wid; k < slots; k += nw) {
+            const int L = k * ctas + rank;
+            if (L >= N) continue;
+            const double A[3] = {Pn[3 * L], Pn[3 * L + 1], Pn[3 * L + 2]};
+            const int cA = Cn[L];
+            int ncand = S.cdc[k];
+            if (s == 0 || (flags & 1)) {
+                ncand = 0;
+                const double cut = (2.4 + kSkin) * m.rad;
+                for (int b = 0; b < N; b += 32) {
+                    const int P = b + lane;
+                    const bool in = P < N && P != L && box_dist2(m, A, Pn + 3 * P) < cut * cut;
+                    const unsigned bal = __ballot_sync(0xffffffffu, in);
+                    const int at = ncand + __popc(bal & ((1u << lane) - 1u));
+                    if (in && at < kMaxCand) S.cand[k * kMaxCand + at] = (unsigned short)P;
+                    ncand += __popc(bal);
+                }
+                if (ncand > kMaxCand) ncand = 255;   // too many to keep: every particle is a candidate
+                if (lane == 0) S.cdc[k] = (unsigned char)ncand;
+                if (lane < 3) S.pcand[3 * k + lane] = Pn[3 * L + lane];
+                __syncwarp();
+            }
+            const bool all = ncand == 255;
+            const int n = all ? N : ncand;
+            int nown = 0, nmir = 0;
+            for (int b = 0; b < n; b += 32) {
+                const int at = b + lane;
+                int P = -1, o = 27;
+                if (at < n) P = all ? at : S.cand[k * kMaxCand + at];
+                if (P >= 0 && P != L)
+                    o = P > L ? first_image(m, A, cA, Pn + 3 * P, Cn[P]) : first_image(m, Pn + 3 * P, Cn[P], A, cA);
+                const unsigned bo = __ballot_sync(0xffffffffu, o < 27 && P > L), bm = __ballot_sync(0xffffffffu, o < 27 && P < L);
+                const unsigned below = (1u << lane) - 1u;
+                if (o < 27 && P > L) { const int q = nown + __popc(bo & below); if (q < kMaxList) { W.own[q] = (unsigned short)P; W.key[q] = (unsigned short)o; } }
+                if (o < 27 && P < L) { const int q = nmir + __popc(bm & below); if (q < kMaxList) W.mir[q] = (unsigned short)P; }
+                nown += __popc(bo);
+                nmir += __popc(bm);
+            }
+            __syncwarp();
+            if (nmir + 1 + nown + 1 > MX) {   // MX < kMaxList: the scratch lists were long enough
+                if (lane == 0) { atomicCAS(&sc->status, 0, PIBM_ERR_NEIGH_OVERFLOW); raise(2, (s + 1) % 3); }
+                continue;
+            }
+            for (int q = lane; q < nmir; q += 32) S.nb[k * MX + q] = W.mir[q];   // ascending
+            for (int q = lane; q < nown; q += 32) {   // by scan offset, ascending within a cell
+                const int o = W.key[q];
+                int r = 0;
+                for (int e = 0; e < nown; ++e) r += W.key[e] < o || (W.key[e] == o && e < q) ? 1 : 0;
+                S.nb[k * MX + nmir + 1 + r] = W.own[q];
+            }
+            if (lane == 0) { S.nb[k * MX + nmir] = (unsigned short)L; S.nbc[k] = (unsigned char)(nmir + 1 + nown); }
+            __syncwarp();
+        }
+    }
+    // the last sub-step's state back to global memory, where the other kernels and the next step read it
+    for (int k = wid; k < slots && s > 0; k += nw) {
+        const int L = k * ctas + rank;
+        if (L >= N) continue;
+        if (lane < 3) {
+            m.pos[3 * L + lane] = m.pos_old[3 * L + lane] = S.P[c][3 * L + lane];
+            m.vel[3 * L + lane] = m.vel_old[3 * L + lane] = S.V[c][3 * L + lane];
+            m.pijk[3 * L + lane] = cell_dir(S.cell[c][L], lane);
+        }
+        const int nc = S.nbc[k], pc = S.pcs[c * slots + k];
+        for (int q = lane; q < nc; q += 32) m.neigh[L * MX + q] = S.nb[k * MX + q];
+        if (c)
+            for (int q = lane; q < pc; q += 32) { m.pn[L * MX + q] = __ldcg(m.pn2 + L * MX + q); m.pv[L * MX + q] = __ldcg(m.pv2 + L * MX + q); }
+        if (lane == 0) { m.ncnt[L] = nc; m.pncnt[L] = pc; }
+    }
+    cl.sync();   // no CTA leaves while another may still store into its copy
 }
 
 // IBMUPDATE (collision_mod.F90:1464-1474): grid-unit centres and velocities.
@@ -802,13 +1152,46 @@ void enqueue_moving_scalar_t(const Geo &g, const Mov &m, Scal *sc, cudaStream_t 
     k_ssp_count<N><<<(g.nsev + 255) / 256, 256, 0, s>>>(g, m, sc);
 }
 
+// Shape of the sub-step kernel: CTAs of few warps each up to the cluster's 8
+// (FP64 instructions of one SM's warps queue on its pipes: 43 particles on two
+// CTAs took 6.3 us per sub-step), and a warp per particle as far as shared
+// memory holds the warps' scratch.
+struct MarchShape { int ctas, warps; size_t smem; };
+MarchShape march_shape(const Mov &m) {
+    MarchShape t;
+    t.ctas = std::min(kMarchCtas, (m.N + 3) / 4);
+    const int slots = (m.N + t.ctas - 1) / t.ctas;
+    t.warps = std::min(32, slots);
+    while (t.warps > 1 && MarchMem::bytes(m.N, slots, m.maxn, t.warps) > 227 * 1024) --t.warps;
+    t.smem = MarchMem::bytes(m.N, slots, m.maxn, t.warps);
+    return t;
+}
+bool use_march(const Mov &m) { return m.soft && m.N <= kMarchMax && m.maxn < kMaxList && m.cx < 1024 && m.cy < 1024 && m.cz < 1024; }
+void launch_march(const Mov &m, Scal *sc, const double *pres, const double *visc, cudaStream_t s) {
+    const MarchShape t = march_shape(m);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)t.ctas, 1, 1);
+    cfg.blockDim = dim3((unsigned)(32 * t.warps), 1, 1);
+    cfg.dynamicSmemBytes = t.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)t.ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_dem_march, m, sc, pres, visc);
+}
+
 template <int N>
 void enqueue_moving_t(const Geo &g, const Mov &m, Scal *sc, const double *pres, const double *visc, cudaStream_t s) {
     const int pb = (m.N + 127) / 128;
     k_dem_start<<<1, 32, 0, s>>>(m, sc);
     if (m.soft) {
         const size_t bin_smem = (size_t)(3 * m.ncell + 1 + m.N) * sizeof(int);
-        for (int ifac = 1; ifac <= m.max_factor; ++ifac) {
+        if (use_march(m)) launch_march(m, sc, pres, visc, s);
+        else for (int ifac = 1; ifac <= m.max_factor; ++ifac) {
             k_dem_update<<<(m.N + kUpdWarps - 1) / kUpdWarps, 32 * kUpdWarps, 0, s>>>(m, sc, pres, visc, ifac);
             k_dem_bin<<<1, 1024, bin_smem, s>>>(m, sc, ifac);
             k_dem_search<<<(m.N + kSearchWarps - 1) / kSearchWarps, 32 * kSearchWarps, 0, s>>>(m, sc, ifac);
@@ -839,7 +1222,7 @@ void enqueue_moving(const Geo &g, const Mov &m, Scal *sc, const double *pres, co
         case 256: enqueue_moving_t<256>(g, m, sc, pres, visc, s); break;
     }
 }
-int moving_kernels_per_step(const Mov &m) { return 1 + (m.soft ? 3 * m.max_factor : 1) + 6; }
+int moving_kernels_per_step(const Mov &m) { return 1 + (m.soft && !use_march(m) ? 3 * m.max_factor : 1) + 6; }
 
 // Scalar geometry of the step (before calc_inner_rev_data) and its spreading.
 void enqueue_moving_scalar(const Geo &g, const Mov &m, Scal *sc, cudaStream_t s) {
@@ -873,6 +1256,8 @@ void enqueue_dem_init(const Mov &m, Scal *sc, cudaStream_t s) {
 
 cudaError_t configure_moving_kernels(const Mov &m) {
     const int smem = (int)((size_t)(3 * m.ncell + 1 + m.N) * sizeof(int));
+    const cudaError_t e = cudaFuncSetAttribute(k_dem_march, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_dem_bin, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 

@@ -139,3 +139,24 @@ def test_moving_with_passive_scalar_matches_oracle():
     assert rel(sg["flux_body"], sc["flux_body"]) <= TOL
     assert abs(sg["heat_ratio"] - sc["heat_ratio"]) <= TOL * abs(sc["heat_ratio"])
     assert abs(rg["nusselt"] - rc["nusselt"]) <= TOL * abs(rc["nusselt"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("my,dia,n,spread", [(32, 10.0, 1, 0.1), (32, 10.0, 5, 3.0), (32, 8.0, 31, 0.5), (64, 12.0, 40, 12.0),
+                                             (64, 8.0, 100, 1.0), (64, 6.0, 512, 2.0), (64, 6.0, 513, 2.0)])
+def test_dem_lists_over_particle_counts(my, dia, n, spread):
+    """The one-launch DEM (up to 512 spheres) and the launches per sub-step
+    (513): one sphere, fewer than the cluster's warps, more than one per warp,
+    boxes of two and three coarse cells (an image of a sphere through several
+    cells), and spheres fast enough that the candidate lists are rebuilt within a step."""
+    rng = np.random.default_rng(n)
+    prm, _ = config.single_sphere(my=my, dia_cells=dia, re=20.0)
+    prm.update(imove=1, collision_type="softsphere", rhos=100.0, rhof=1.0, coeff_rest=0.9, initialize_zero=True)
+    xc = config.fcc_subset(n, float(my), dia, rng)
+    xc, _ = config.hard_sphere_mc(xc, float(my), dia, rng, 4 * n, 0.1 * dia)
+    vel = rng.normal(0.0, spread * 20.0 * prm["vis"], size=xc.shape)
+    gpu, cpu = make_pair(prm, xc, vel - vel.mean(axis=0, keepdims=True) * (n > 1))
+    for _ in range(2):
+        gpu.step()
+        cpu.step()
+        compare(gpu, cpu)
