@@ -192,8 +192,7 @@ static int setup_moving(pibm_handle *h) {
     if (!ok) return rc;
     if (g.scal) {
         ok = guard(h->alloc(&m.sev_cnt, (size_t)N), "sev counts") && guard(h->alloc(&m.sev_off, (size_t)N), "sev offsets") &&
-             guard(h->alloc(&m.sspcnt, nodes), "scalar spread counts") &&
-             guard(h->alloc(&m.sspbuf, nodes * (size_t)m.kmax), "scalar spread buckets");
+             guard(h->alloc(&m.sev_of, (size_t)N * S.nbnd), "sev of points");
         if (!ok) return rc;
         m.sev_m = const_cast<int *>(g.sev_m); m.sev_l = const_cast<int *>(g.sev_l);
         m.sev_c = const_cast<int *>(g.sev_c); m.sev_x = const_cast<double *>(g.sev_x);

@@ -96,10 +96,10 @@ struct Mov {
     int *spcnt, *spbuf;                        // spreading buckets: count and entries per node
     int kmax;                                  // bucket capacity per node
     // passive scalar with moving particles: reversal-point evaluations per
-    // sphere and in total, and the scalar forcing's spreading buckets
+    // sphere and in total
     int *sev_cnt, *sev_off, *sev_m, *sev_l, *sev_c;
     double *sev_x;
-    int *sspcnt, *sspbuf;
+    int *sev_of;                               // per active point: its first evaluation, ~index when it has two
 };
 
 // Device buffers of one run.

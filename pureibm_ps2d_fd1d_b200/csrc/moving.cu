@@ -951,9 +951,11 @@ __global__ void __launch_bounds__(256) k_sp_count(Geo g, Mov m, Scal *sc) {
 template <class F>
 __device__ __forceinline__ void bucket_in_order(const int *bucket, int c, F f) {
     if (c <= 8) {
-        int v[8];
+        // whole 16-byte loads (a bucket holds kmax >= 8 slots at a 64-byte multiple)
+        const int4 lo = *(const int4 *)bucket, hi = c > 4 ? *(const int4 *)(bucket + 4) : make_int4(0, 0, 0, 0);
+        int v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = q < c ? bucket[q] : 0x7fffffff;
+        for (int q = 0; q < 8; ++q) v[q] = q < c ? v[q] : 0x7fffffff;
         auto ce = [&](int a, int b) { const int x = min(v[a], v[b]), y = max(v[a], v[b]); v[a] = x; v[b] = y; };
         ce(0, 1); ce(2, 3); ce(4, 5); ce(6, 7);
         ce(0, 2); ce(1, 3); ce(4, 6); ce(5, 7);
@@ -977,31 +979,68 @@ __device__ __forceinline__ void bucket_in_order(const int *bucket, int c, F f) {
     }
 }
 
+// The forced nodes of a block's window of kSpreadWin consecutive nodes, dense
+// over its threads.  Forced nodes are a shell around each sphere, and the
+// transform order deals neighbouring nodes to different warps, so one thread
+// per node left a warp with a few forced lanes that the others waited for.
+// none(node) is called for every node without entries, by consecutive threads;
+// some(node, entries) for the others.  Nodes are independent: their order
+// among the threads does not matter.
+// 256^3, 1202 spheres: k_spread_dyn 1.49 -> 0.81 ms.
+constexpr int kSpreadWin = 1024;
+template <class F0, class F1>
+__device__ __forceinline__ void for_forced_nodes(const int *cnt, size_t nodes, int kmax, F0 none, F1 some) {
+    __shared__ unsigned short list[kSpreadWin], num[kSpreadWin];
+    __shared__ int total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    const size_t base = (size_t)blockIdx.x * kSpreadWin;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < kSpreadWin; k += 256) {
+        const size_t node = base + k + threadIdx.x;
+        const int c = node < nodes ? cnt[node] : 0;
+        if (node < nodes && c == 0) none(node);
+        const unsigned bal = __ballot_sync(0xffffffffu, c > 0);
+        int at = 0;
+        if (lane == 0 && bal) at = atomicAdd(&total, __popc(bal));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
+        if (c > 0) { list[at] = (unsigned short)(k + threadIdx.x); num[at] = (unsigned short)min(c, kmax); }
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < total; q += blockDim.x) some(base + list[q], (int)num[q]);
+}
+
 // fr at every node: the bucket's contributions in ascending (point, corner)
 // order, the reference's accumulation order; nodes without force get zero.
 __global__ void __launch_bounds__(256) k_spread_dyn(Geo g, Mov m, const double *__restrict__ rec,
                                                     const double *__restrict__ rz, double *__restrict__ fr, Scal *sc) {
-    const size_t node = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t CR = (size_t)g.nx * g.RS;
-    if (node >= CR || sc->status) return;
+    if (block_failed(sc)) return;
     const double rdx3 = 1.0 / g.dx3;
-    double acc[3] = {0.0, 0.0, 0.0};
-    const int c = min(m.spcnt[node], m.kmax);
-    if (c > 0)
-        bucket_in_order(m.spbuf + node * m.kmax, c, [&](int ent) {
-            double t[3];
-            corner_contrib(rz, rec, ent, g.dx3, rdx3, t);
-            if (g.include_frmeanfluid) {
+    for_forced_nodes(
+        m.spcnt, CR, m.kmax,
+        [&](size_t node) {
 #pragma unroll
-                for (int n = 0; n < 3; ++n) acc[n] = acc[n] + t[n];
-            } else {
-                const double *r = rec + (size_t)(ent >> 3) * 6 + 3;
+            for (int n = 0; n < 3; ++n) fr[n * CR + node] = 0.0;
+        },
+        [&](size_t node, int c) {
+            double acc[3] = {0.0, 0.0, 0.0};
+            bucket_in_order(m.spbuf + node * m.kmax, c, [&](int ent) {
+                double t[3];
+                corner_contrib(rz, rec, ent, g.dx3, rdx3, t);
+                if (g.include_frmeanfluid) {
 #pragma unroll
-                for (int n = 0; n < 3; ++n) acc[n] = (acc[n] + t[n]) + r[n];
-            }
+                    for (int n = 0; n < 3; ++n) acc[n] = acc[n] + t[n];
+                } else {
+                    const double *r = rec + (size_t)(ent >> 3) * 6 + 3;
+#pragma unroll
+                    for (int n = 0; n < 3; ++n) acc[n] = (acc[n] + t[n]) + r[n];
+                }
+            });
+#pragma unroll
+            for (int n = 0; n < 3; ++n) fr[n * CR + node] = acc[n];
         });
-#pragma unroll
-    for (int n = 0; n < 3; ++n) fr[n * CR + node] = acc[n];
 }
 
 // ---------------------------------------------------------------------------
@@ -1072,26 +1111,29 @@ __global__ void __launch_bounds__(1024) k_sev_scan(Geo g, Mov m, Scal *sc) {
     if (t == T - 1) sc->nsev = run;
 }
 
-// One sphere's evaluations written in (point, evaluation) order at its offset.
+// One sphere's evaluations written in (point, evaluation) order at its offset,
+// and for every active point the index of its first one (negated: ~index, when it has two).
 __global__ void __launch_bounds__(256) k_sev_write(Geo g, Mov m, Scal *sc) {
-    __shared__ int wsum[8];
-    __shared__ int base;
+    __shared__ int wsum[8], wact[8];
+    __shared__ int base, pbase;
     if (block_failed(sc)) return;
     const int s = blockIdx.x, nb = g.nbnd, t = threadIdx.x, lane = t & 31, wid = t >> 5, mxf = g.nx + 1;
-    if (t == 0) base = m.sev_off[s];
+    if (t == 0) { base = m.sev_off[s]; pbase = m.ptoff[s]; }
     __syncthreads();
     for (int l0 = 0; l0 < nb; l0 += blockDim.x) {
         const int l = l0 + t;
         ScalEval e;
         int n = 0;
         if (l < nb && m.revflag[(size_t)s * nb + l]) { e = scal_eval(g, m, s, l); n = e.nev; }
+        const unsigned act = __ballot_sync(0xffffffffu, n > 0);
         int x = n;
         for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
-        if (lane == 31) wsum[wid] = x;
+        if (lane == 31) { wsum[wid] = x; wact[wid] = __popc(act); }
         __syncthreads();
-        int before = 0;
-        for (int w = 0; w < wid; ++w) before += wsum[w];
+        int before = 0, pbefore = 0;
+        for (int w = 0; w < wid; ++w) { before += wsum[w]; pbefore += wact[w]; }
         int q = base + before + x - n;
+        if (n > 0) m.sev_of[pbase + pbefore + __popc(act & ((1u << lane) - 1u))] = n == 2 ? ~q : q;
         for (int ev = 1; ev <= n; ++ev, ++q) {
             if (ev == 2 && e.c[0] >= mxf - 1) { e.c[0] = e.c[0] - (mxf - 1); e.x[0] = e.x[0] - (mxf - 1); }
             m.sev_m[q] = s;
@@ -1100,47 +1142,35 @@ __global__ void __launch_bounds__(256) k_sev_write(Geo g, Mov m, Scal *sc) {
             for (int d = 0; d < 3; ++d) { m.sev_x[3 * (size_t)q + d] = e.x[d]; m.sev_c[3 * (size_t)q + d] = e.c[d]; }
         }
         __syncthreads();
-        if (t == 0) { int a = 0; for (int w = 0; w < (int)(blockDim.x >> 5); ++w) a += wsum[w]; base += a; }
+        if (t == 0)
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { base += wsum[w]; pbase += wact[w]; }
         __syncthreads();
     }
 }
 
-// Scalar spreading targets: stencil corners on planes 1..nx (planes 0 and
-// nx+1 are never transformed), solid nodes unless INCLUDE_FRMEANFLUID.
-template <int N>
-__global__ void __launch_bounds__(256) k_ssp_count(Geo g, Mov m, Scal *sc) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sc->status || e >= sc->nsev) return;
-    const int nx = g.nx, mxf = g.nx + 1;
-    const int c0 = m.sev_c[3 * (size_t)e], c1 = m.sev_c[3 * (size_t)e + 1], c2 = m.sev_c[3 * (size_t)e + 2];
-    for (int ck = 0; ck < 2; ++ck)
-        for (int cj = 0; cj < 2; ++cj)
-            for (int ci = 0; ci < 2; ++ci) {
-                int i = c0 + ci;
-                if (i < 0) i = mxf + i - 1;
-                if (i < 1 || i > nx) continue;
-                const int j = wrapi(c1 + cj, N), k = wrapi(c2 + ck, N);
-                const size_t node = (size_t)(i - 1) * RP<N>::RSP + real_off<N>(k - 1, j - 1);
-                if (!g.include_frmeanfluid && m.fluid[node]) continue;
-                const int slot = atomicAdd(&m.sspcnt[node], 1);
-                if (slot < m.kmax) m.sspbuf[node * m.kmax + slot] = e * 8 + ci + 2 * cj + 4 * ck;
-                else atomicCAS(&sc->status, 0, PIBM_ERR_SPREAD_OVERFLOW);
-            }
-}
-
-// Scalar forcing at every node of planes 1..nx in (evaluation, corner) order.
+// Scalar forcing at every node of planes 1..nx in (evaluation, corner) order,
+// from the flow's buckets: a point's evaluations put its 8 stencil corners on
+// the nodes its point force goes to (the corners of cell nx's second plane come
+// from the second evaluation, one period west; corners off planes 1..nx are
+// dropped by one evaluation and covered by the other), and evaluations are
+// numbered in point order, so a bucket in (point, corner) order is in
+// (evaluation, corner) order too.  Buckets of its own (k_ssp_count) took 0.33 ms
+// per step and 2.1 GB at 256^3.
 __global__ void __launch_bounds__(256) k_sspread_dyn(Geo g, Mov m, const double *__restrict__ sctb,
                                                      const double *__restrict__ sfd, double *__restrict__ sfr, Scal *sc) {
-    const size_t node = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (node >= (size_t)g.nx * g.RS || sc->status) return;
-    double v = 0.0;
-    const int c = min(m.sspcnt[node], m.kmax);
-    if (c > 0)
-        bucket_in_order(m.sspbuf + node * m.kmax, c, [&](int ent) {
-            v = v + sctb[ent];
-            if (!g.include_frmeanfluid) v = v + sfd[ent >> 3];
+    if (block_failed(sc)) return;
+    for_forced_nodes(
+        m.spcnt, (size_t)g.nx * g.RS, m.kmax, [&](size_t node) { sfr[node] = 0.0; },
+        [&](size_t node, int c) {
+            double v = 0.0;
+            bucket_in_order(m.spbuf + node * m.kmax, c, [&](int ent) {
+                const int f = m.sev_of[ent >> 3];
+                const size_t e = (size_t)(f >= 0 ? f : ~f + (ent & 1));   // corner bit 0: the second x plane
+                v = v + sctb[8 * e + (ent & 7)];
+                if (!g.include_frmeanfluid) v = v + sfd[e];
+            });
+            sfr[node] = v;
         });
-    sfr[node] = v;
 }
 
 template <int N>
@@ -1148,8 +1178,6 @@ void enqueue_moving_scalar_t(const Geo &g, const Mov &m, Scal *sc, cudaStream_t 
     k_sev_count<<<g.nbody, 256, 0, s>>>(g, m, sc);
     k_sev_scan<<<1, 1024, 0, s>>>(g, m, sc);
     k_sev_write<<<g.nbody, 256, 0, s>>>(g, m, sc);
-    cudaMemsetAsync(m.sspcnt, 0, (size_t)g.nx * RP<N>::RSP * sizeof(int), s);
-    k_ssp_count<N><<<(g.nsev + 255) / 256, 256, 0, s>>>(g, m, sc);
 }
 
 // Shape of the sub-step kernel: CTAs of few warps each up to the cluster's 8
@@ -1236,13 +1264,13 @@ void enqueue_moving_scalar(const Geo &g, const Mov &m, Scal *sc, cudaStream_t s)
 }
 void enqueue_sspread_dyn(const Geo &g, const Mov &m, const double *sctb, const double *sfd, double *sfr, Scal *sc, cudaStream_t s) {
     const size_t CR = (size_t)g.nx * g.RS;
-    k_sspread_dyn<<<(unsigned)((CR + 255) / 256), 256, 0, s>>>(g, m, sctb, sfd, sfr, sc);
+    k_sspread_dyn<<<(unsigned)((CR + kSpreadWin - 1) / kSpreadWin), 256, 0, s>>>(g, m, sctb, sfd, sfr, sc);
 }
-int moving_scalar_kernels_per_step() { return 4; }
+int moving_scalar_kernels_per_step() { return 3; }
 
 void enqueue_spread_dyn(const Geo &g, const Mov &m, const double *rec, const double *rz, double *fr, Scal *sc, cudaStream_t s) {
     const size_t CR = (size_t)g.nx * g.RS;
-    k_spread_dyn<<<(unsigned)((CR + 255) / 256), 256, 0, s>>>(g, m, rec, rz, fr, sc);
+    k_spread_dyn<<<(unsigned)((CR + kSpreadWin - 1) / kSpreadWin), 256, 0, s>>>(g, m, rec, rz, fr, sc);
 }
 
 // Set-up: cells and the first neighbour search of des_time_march(.TRUE.)
