@@ -546,11 +546,14 @@ __device__ __forceinline__ double slope_d(double um1, double u0, double up1, dou
 // each face's partials are formed once and added to a rolling window of the
 // four cells it reads; a cell is complete once the face after it is done.
 // ============================================================================
-constexpr int kAdjFluxSeg = 16;   // x cells per thread (divides every supported nx)
+// x cells per thread (divides every supported nx): a segment forms 3 faces
+// beyond its own, but 16 cells leave a 96^3 grid 1.5 blocks per SM
+// (110 -> 96 us with 8).
+__host__ __device__ constexpr int adj_flux_seg(int n) { return n <= 64 ? 4 : n <= 96 ? 8 : 16; }
 template <int N>
 __global__ void __launch_bounds__(256) k_adj_flux(Geo g, const double *__restrict__ ubcp, const double *__restrict__ W8,
                                                   double *lubcp) {
-    constexpr int RSP = RP<N>::RSP, SEG = kAdjFluxSeg;
+    constexpr int RSP = RP<N>::RSP, SEG = adj_flux_seg(N);
     const int nx = g.nx, nseg = nx / SEG;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= RSP * nseg) return;
@@ -706,7 +709,7 @@ static void enqueue_adjoint_step_t(const Geo &g, const DevBufs &b, const AdjBufs
     launch_planes<RL<N>>(k_adj_r2c<N>, 3 * g.nx, 1, s, g, (const double *)a.lQ, a.T, a.as);
     k_adj_q<<<(unsigned)((3 * SC + 255) / 256), 256, 0, s>>>(g, a.T, a.lnl_new, a.lonl, a.lu2);
     launch_planes<PL<N>>(k_adj_c2r<N>, g.nx, 8, s, g, (const double2 *)a.lnl_new, a.W8, 1);
-    k_adj_flux<N><<<(unsigned)((RP<N>::RSP * (g.nx / kAdjFluxSeg) + 255) / 256), 256, 0, s>>>(g, b.ubcp, a.W8, a.lubcp);
+    k_adj_flux<N><<<(unsigned)((RP<N>::RSP * (g.nx / adj_flux_seg(N)) + 255) / 256), 256, 0, s>>>(g, b.ubcp, a.W8, a.lubcp);
     k_adj_sum<N><<<dim3(nsum, 3), 256, 0, s>>>(g, a.lubcp, lumean, 1.0);
     launch_planes<RL<N>>(k_adj_r2c<N>, 10 * g.nx, 1, s, g, (const double *)a.lubcp, a.T, a.as);
     k_adj_assemble<<<(unsigned)((SC + 255) / 256), 256, 0, s>>>(g, a.T, a.lu2, a.lp2);

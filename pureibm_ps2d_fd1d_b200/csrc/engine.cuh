@@ -142,12 +142,12 @@ struct MemberSet {
 };
 
 // Planes one thread of k_flux marches through (a sliding window along x; a
-// segment re-reads two planes on either side).  Short segments give grids up
-// to 128^3 enough threads to keep loads in flight when the flux is on the
-// step's critical path (k_flux 41 -> 35 us at 128^3); with the passive
-// scalar's kernels running beside it the GPU is full, and long segments, which
-// re-read less, give the shorter step.
-inline int flux_segment(int n, bool scalar) { return (scalar || n >= 256) ? 32 : 8; }
+// segment re-reads two planes on either side).  Short segments give small
+// grids enough threads to keep loads in flight when the flux is on the step's
+// critical path: k_flux 12.7 -> 8.6 us at 32, 12.7 -> 10.7 at 64 with 2 planes
+// instead of 8 (no gain at 96), 41 -> 35 at 128 with 8 instead of 32.  With the passive scalar's kernels running beside it the GPU
+// is full from 128^3 on, and long segments, which re-read less, give the shorter step.
+inline int flux_segment(int n, bool scalar) { return n <= 64 ? 2 : (scalar && n >= 128) || n >= 256 ? 32 : 8; }
 
 // Launch extents of a fused batch step: runs in the group and the largest
 // sphere count, reversal-forcing block count and spreading node count among

@@ -791,6 +791,49 @@ __device__ __forceinline__ void b_spread(const Geo &g, const double *__restrict_
 }
 __global__ void __launch_bounds__(256) k_spread(Geo g, const double *__restrict__ rec, const double *__restrict__ rz,
                                                 double *__restrict__ fr, const Scal *__restrict__ sc) { b_spread(g, rec, rz, fr, sc); }
+// The same sums with kSpreadLanes lanes per node: the lanes form that many
+// contributions at once and every lane adds them in the list's order, so the
+// result is bitwise b_spread's.  For launches of few nodes, which are as
+// long as the longest list: each of its contributions is two dependent trips
+// to L2 (23 -> 10.6 us at 32^3 with 4 k nodes, 18 -> 9 us for one
+// sphere at 64^3; no gain with 37 k nodes, 23 -> 27 us with 60 k).
+constexpr int kSpreadLanes = 8;
+constexpr long long kSpreadFewNodes = 20000;
+__device__ __forceinline__ void b_spread_lanes(const Geo &g, const double *__restrict__ rec, const double *__restrict__ rz,
+                                               double *__restrict__ fr, const Scal *__restrict__ sc) {
+    constexpr int G = kSpreadLanes;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, q = t / G, sub = t % G;
+    if (block_failed(sc)) return;
+    const bool in = q < g.sp_nnodes;
+    const int e0 = in ? g.sp_ptr[q] : 0, e1 = in ? g.sp_ptr[q + 1] : 0;
+    const int rounds = __reduce_max_sync(0xffffffffu, (unsigned)(e1 - e0 + G - 1) / G);
+    const double rdx3 = 1.0 / g.dx3;
+    double acc[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < rounds; ++k) {
+        const int e = e0 + k * G + sub;
+        double c[3] = {0.0, 0.0, 0.0}, r[3] = {0.0, 0.0, 0.0};
+        if (e < e1) {
+            const int ent = __ldg(g.sp_ent + e);
+            corner_contrib(rz, rec, ent, g.dx3, rdx3, c);
+            if (!g.include_frmeanfluid)
+#pragma unroll
+                for (int n = 0; n < 3; ++n) r[n] = __ldg(rec + (size_t)(ent >> 3) * 6 + 3 + n);
+        }
+#pragma unroll
+        for (int j = 0; j < G; ++j)
+#pragma unroll
+            for (int n = 0; n < 3; ++n) {
+                const double cj = __shfl_sync(0xffffffffu, c[n], j, G), rj = __shfl_sync(0xffffffffu, r[n], j, G);
+                if (e0 + k * G + j < e1) {
+                    acc[n] = acc[n] + cj;
+                    if (!g.include_frmeanfluid) acc[n] = acc[n] + rj;
+                }
+            }
+    }
+    if (in && sub < 3) fr[sub * (size_t)g.nx * g.RS + g.sp_node[q]] = sub == 0 ? acc[0] : sub == 1 ? acc[1] : acc[2];
+}
+__global__ void __launch_bounds__(256) k_spread_lanes(Geo g, const double *__restrict__ rec, const double *__restrict__ rz,
+                                                      double *__restrict__ fr, const Scal *__restrict__ sc) { b_spread_lanes(g, rec, rz, fr, sc); }
 
 // k_ff: ff = r2c(fr - frmean) (boundary_condition.F90:678-700).
 template <int N>
@@ -1287,6 +1330,11 @@ __global__ void __launch_bounds__(256) kb_spread(const __grid_constant__ MemberS
     if (m.g.nbody == 0 || m.g.npts == 0) return;
     b_spread(m.g, m.b.rec, m.b.rz, m.b.fr, m.b.sc);
 }
+__global__ void __launch_bounds__(256) kb_spread_lanes(const __grid_constant__ MemberSet ms) {
+    const Member &m = ms.m[blockIdx.z];
+    if (m.g.nbody == 0 || m.g.npts == 0) return;
+    b_spread_lanes(m.g, m.b.rec, m.b.rz, m.b.fr, m.b.sc);
+}
 template <int N>
 __global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) kb_ff(const __grid_constant__ MemberSet ms) {
     const Member &m = ms.m[blockIdx.z];
@@ -1333,7 +1381,11 @@ static void enqueue_batch_step_t(const MemberSet &ms, const BatchShape &bs, cuda
             cudaStreamWaitEvent(side, fork, 0);
             kb_scal_c<<<dim3(1, 1, nz), 256, 0, side>>>(ms);
             cudaEventRecord(join, side);
-            if (bs.max_spn > 0) kb_spread<<<dim3((bs.max_spn + 255) / 256, 1, nz), 256, 0, s>>>(ms);
+            if (bs.max_spn > 0) {
+                if ((long long)bs.max_spn * nz <= kSpreadFewNodes)
+                    kb_spread_lanes<<<dim3((bs.max_spn * kSpreadLanes + 255) / 256, 1, nz), 256, 0, s>>>(ms);
+                else kb_spread<<<dim3((bs.max_spn + 255) / 256, 1, nz), 256, 0, s>>>(ms);
+            }
             cudaStreamWaitEvent(s, join, 0);
         }
         launch_planes_z<RL<N>>(kb_ff<N>, N, 3, nz, s, ms);
@@ -1518,7 +1570,8 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
             }
             kb(PIBM_K_SPREAD);
             if (g.moving) enqueue_spread_dyn(g, b.mov, b.rec, b.rz, b.fr, b.sc, s);
-            else if (g.sp_nnodes > 0) k_spread<<<(g.sp_nnodes + 255) / 256, 256, 0, s>>>(g, b.rec, b.rz, b.fr, b.sc);
+            else if (g.sp_nnodes > kSpreadFewNodes) k_spread<<<(g.sp_nnodes + 255) / 256, 256, 0, s>>>(g, b.rec, b.rz, b.fr, b.sc);
+            else if (g.sp_nnodes > 0) k_spread_lanes<<<(g.sp_nnodes * kSpreadLanes + 255) / 256, 256, 0, s>>>(g, b.rec, b.rz, b.fr, b.sc);
             ke(PIBM_K_SPREAD);
             if (fork && !scal_first) cudaStreamWaitEvent(s, ss->frmean_done, 0);
         } else {

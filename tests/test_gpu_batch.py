@@ -99,3 +99,29 @@ def test_mixed_batch_matches_single_runs_bitwise(fused):
         assert got["t"] == want["t"] and got["dt"] == want["dt"]
         s.close()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("my,dia,n,width,limiter,frfl", [(32, 8.0, 1, 2, "none", False), (32, 8.0, 3, 12, "minmod", True),
+                                                         (64, 10.0, 1, 10, "none", False), (64, 7.0, 40, 2, "none", False)])
+def test_spreading_by_lanes_equals_one_thread_per_node_bitwise(my, dia, n, width, limiter, frfl):
+    """Launches of few forced nodes spread with several lanes per node, the
+    others with one thread: a narrow batch and its members alone take the
+    former, a wide batch and an array of 40 spheres the latter, and every
+    combination ends at the same bits."""
+    if n == 1:
+        prm, xc = config.single_sphere(my=my, dia_cells=dia)
+    else:
+        prm, xc = config.random_array(my=my, dia_cells=dia, nbody=n, seed=n, mc_moves=20)
+    prm.update(limiter=limiter, include_frmeanfluid=frfl)
+    b = pk.Batch([(dict(prm), xc)] * width)
+    b.run(3)
+    s = pk.Solver(prm, xc)
+    s.run(3)
+    want = s.get_state()
+    for q in (0, width - 1):
+        got = b.members[q].get_state()
+        for k in ("u", "nl", "p"):
+            np.testing.assert_array_equal(got[k], want[k])
+    s.close()
+    b.close()
