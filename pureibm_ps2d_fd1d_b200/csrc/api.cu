@@ -27,13 +27,13 @@ void enqueue_step(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cudaEvent_t
 int kernels_per_step(const Geo &g, const Mov &m);
 void enqueue_batch_step(int n, const MemberSet &ms, const BatchShape &bs, cudaStream_t s, cudaStream_t side,
                         cudaEvent_t fork, cudaEvent_t join);
-int batch_kernels_per_step(const BatchShape &bs);
 void enqueue_dem_init(const Mov &m, Scal *sc, cudaStream_t s);
 cudaError_t configure_moving_kernels(const Mov &m);
 void enqueue_c2r(const Geo &g, const double2 *a, double *b, int nplanes, cudaStream_t s);
 void enqueue_r2c(const Geo &g, const double *a, double2 *b, int nplanes, cudaStream_t s);
 void enqueue_f2d(const double2 *f, double2 *d, int nx, int nxf, int PS, int ncomp, cudaStream_t s);
-void enqueue_d2f(const double2 *d, double2 *f, int nx, int nxf, int PS, int ncomp, cudaStream_t s);
+void enqueue_d2f(const double2 *d, double2 *f, int nx, int nxf, int PS, int ncomp, cudaStream_t s, const double *ratio = nullptr);
+void enqueue_put_scalars(Scal *sc, const Scal &v, cudaStream_t s);
 int real_offset(int n, int z, int y);
 int plane_ctas(int n);
 void enqueue_scalar(const Geo &g, DevBufs &b, int cur, cudaStream_t s);
@@ -84,7 +84,11 @@ struct pibm_handle {
     DevBufs b;
     std::vector<void *> allocs;
     cudaStream_t stream = nullptr;
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};        // a time step per nl parity (pibm_run)
+    cudaGraphExec_t sgraph[3][2] = {};                    // RK3: one stage per rks and nl parity (pibm_step)
+    int step_calls = 0;
+    Scal *hsc = nullptr;        // pinned copy of the device scalars (a pageable one is staged by the driver)
+    double *hpart = nullptr;    // pinned staging of get_particles: pres, visc, ptot, force, xc, vel
     unsigned geo_ver = 0; // bumped whenever the Geo copies change (graphs hold them by value)
     int cur = 0;          // buffer index the next step writes its nonlinear term to
     int device = 0;
@@ -113,6 +117,9 @@ struct pibm_handle {
     }
     ~pibm_handle() {
         for (auto &gx : graph) if (gx) cudaGraphExecDestroy(gx);
+        for (auto &st : sgraph) for (auto &gx : st) if (gx) cudaGraphExecDestroy(gx);
+        if (hsc) cudaFreeHost(hsc);
+        if (hpart) cudaFreeHost(hpart);
         if (stream) cudaStreamDestroy(stream);
         if (ss.side) cudaStreamDestroy(ss.side);
         if (ss.scal) cudaStreamDestroy(ss.scal);
@@ -126,6 +133,7 @@ struct pibm_handle {
 // (recaptured by the next pibm_run; batches compare geo_ver).
 static void drop_graphs(pibm_handle *h) {
     for (auto &gx : h->graph) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
+    for (auto &st : h->sgraph) for (auto &gx : st) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
     ++h->geo_ver;
 }
 
@@ -237,7 +245,7 @@ int pibm_create(const pibm_params *prm, const pibm_particles *parts, pibm_handle
         if (e != cudaSuccess) { rc = fail(PIBM_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)); return false; }
         return true;
     };
-    if (!guard(cudaGetDevice(&h->device), "cudaGetDevice") || !guard(configure_kernels(S.my), "configure_kernels") ||
+    if (!guard(cudaGetDevice(&h->device), "cudaGetDevice") || !guard(cudaMallocHost(&h->hsc, sizeof(Scal)), "pinned scalars") || !guard(configure_kernels(S.my), "configure_kernels") ||
         !guard(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
         !guard(cudaStreamCreateWithFlags(&h->ss.side, cudaStreamNonBlocking), "cudaStreamCreate") ||
         !guard(cudaStreamCreateWithFlags(&h->ss.scal, cudaStreamNonBlocking), "cudaStreamCreate") ||
@@ -307,13 +315,14 @@ int pibm_create(const pibm_params *prm, const pibm_particles *parts, pibm_handle
               guard(h->alloc(&b.omega, 3 * NR), "omega") && guard(h->alloc(&b.pgr, 3 * NR), "pgr") &&
               (S.nbody == 0 || guard(h->alloc(&b.fr, 3 * NR), "fr")) &&
               guard(h->alloc(&b.part, (size_t)g.nx * 8 * 12), "part") &&
-              guard(h->alloc(&b.pres, 3 * (size_t)S.nbody), "pres") && guard(h->alloc(&b.visc, 3 * (size_t)S.nbody), "visc") &&
-              guard(h->alloc(&b.ptot, 3 * (size_t)S.nbody), "ptot") && guard(h->alloc(&b.force, 3 * (size_t)S.nbody), "force") &&
+              guard(h->alloc(&b.pres, 12 * (size_t)S.nbody), "particle forces") &&
               guard(h->alloc(&b.rec, 6 * (size_t)g.npts), "rec") && guard(h->alloc(&b.rz, 3 * (size_t)g.npts), "rz") &&
               guard(h->alloc(&b.dpart, 6 * 8 * (size_t)S.nbody), "dpart") &&
               guard(h->alloc(&b.blockpart, 6 * (size_t)((g.npts + 255) / 256 + 1)), "blockpart") &&
               guard(h->alloc(&b.sc, 1), "scalars");
     if (!ok) { delete h; return rc; }
+    // pres, visc, ptot and force are one block: one copy reads them back
+    b.visc = b.pres + 3 * (size_t)S.nbody; b.ptot = b.visc + 3 * (size_t)S.nbody; b.force = b.ptot + 3 * (size_t)S.nbody;
     if (S.scal) {
         // passive scalar: geometry of the reversal-point evaluations, the
         // spreading map in plane-transform order, and phi = 1 (scalar_init.F90:136-152)
@@ -390,10 +399,17 @@ int pibm_info_get(pibm_handle *h, pibm_info *info) {
     return PIBM_OK;
 }
 
+// The handle's device scalars on the host once its stream has drained.
+static int read_scalars(pibm_handle *h, Scal *sc) {
+    CUDA_OR_FAIL(cudaMemcpyAsync(h->hsc, h->b.sc, sizeof(Scal), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
+    *sc = *h->hsc;
+    return PIBM_OK;
+}
 static int fill_report(pibm_handle *h, pibm_step_report *rep) {
     Scal sc;
-    CUDA_OR_FAIL(cudaMemcpyAsync(&sc, h->b.sc, sizeof(sc), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
+    const int rc = read_scalars(h, &sc);
+    if (rc) return rc;
     if (rep) {
         std::memset(rep, 0, sizeof(*rep));
         rep->dt = sc.dt; rep->t = sc.t; rep->cf = sc.cf; rep->umax = sc.umax;
@@ -421,7 +437,25 @@ int pibm_step(pibm_handle *h, int rks, pibm_step_report *rep) {
     if (!h) return fail(PIBM_ERR_ARG, "null handle");
     if (rks < 1 || rks > h->itrmax) return fail(PIBM_ERR_ARG, h->itrmax == 1 ? "AB2 has a single stage (rks = 1)" : "rks must be 1, 2 or 3 (RK3)");
     if (rks != h->next_rks) return fail(PIBM_ERR_ARG, "stages must run in the order rks = 1..itrmax");
-    enqueue_step(h->gs[rks - 1], h->b, h->cur, h->stream, nullptr, &h->ss);
+    // a host that steps in a loop replays a graph of the stage: its dozen
+    // launches and event waits cost the CPU more than a small grid's step takes
+    // the GPU (the driver loop at 32^3: 181 us per iteration, 118 with the pinned read-backs); the first calls launch directly,
+    // so a few steps do not pay for a capture
+    if (++h->step_calls > 2) {
+        cudaGraphExec_t &gx = h->itrmax == 1 ? h->graph[h->cur] : h->sgraph[rks - 1][h->cur];
+        if (!gx) {
+            cudaGraph_t gr;
+            CUDA_OR_FAIL(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+            enqueue_step(h->gs[rks - 1], h->b, h->cur, h->stream, nullptr, &h->ss);
+            CUDA_OR_FAIL(cudaStreamEndCapture(h->stream, &gr));
+            const cudaError_t e = cudaGraphInstantiate(&gx, gr, 0);
+            cudaGraphDestroy(gr);
+            CUDA_OR_FAIL(e);
+        }
+        CUDA_OR_FAIL(cudaGraphLaunch(gx, h->stream));
+    } else {
+        enqueue_step(h->gs[rks - 1], h->b, h->cur, h->stream, nullptr, &h->ss);
+    }
     CUDA_OR_FAIL(cudaGetLastError());
     h->cur ^= 1;
     h->next_rks = rks == h->itrmax ? 1 : rks + 1;
@@ -554,8 +588,8 @@ int pibm_get_state(pibm_handle *h, pibm_state_view *s) {
         CUDA_OR_FAIL(cudaMemcpyAsync(s->p, tmp, nfp * sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
     }
     Scal sc;
-    CUDA_OR_FAIL(cudaMemcpyAsync(&sc, h->b.sc, sizeof(sc), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
+    const int rc = read_scalars(h, &sc);
+    if (rc) return rc;
     for (int d = 0; d < 3; ++d) { s->umean[d] = sc.umean[d]; s->mpg[d] = sc.mpg[d]; s->ufmean[d] = sc.ufmean[d]; }
     s->t = sc.t; s->dt = sc.dt; s->cf = sc.cf;
     return PIBM_OK;
@@ -581,12 +615,9 @@ int pibm_set_state(pibm_handle *h, const pibm_state_view *s) {
         CUDA_OR_FAIL(cudaMemcpyAsync(tmp, s->p, nfp * sizeof(double2), cudaMemcpyHostToDevice, h->stream));
         enqueue_f2d(tmp, h->b.p, g.nx, g.nx, g.PS, 1, h->stream);
     }
-    Scal sc;
-    CUDA_OR_FAIL(cudaMemcpyAsync(&sc, h->b.sc, sizeof(sc), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
+    Scal sc;   // only the fields enqueue_put_scalars writes
     for (int d = 0; d < 3; ++d) { sc.umean[d] = s->umean[d]; sc.mpg[d] = s->mpg[d]; sc.ufmean[d] = s->ufmean[d]; }
     sc.t = s->t; sc.dt = s->dt; sc.cf = s->cf;
-    sc.status = 0;
     h->next_rks = 1;   // a restart begins a time step
     if (h->g.moving && h->S.dem_soft) {
         // the step graphs hold max_factor DEM sub-steps; a larger dt needs more
@@ -597,7 +628,8 @@ int pibm_set_state(pibm_handle *h, const pibm_state_view *s) {
             drop_graphs(h);
         }
     }
-    CUDA_OR_FAIL(cudaMemcpyAsync(h->b.sc, &sc, sizeof(sc), cudaMemcpyHostToDevice, h->stream));
+    enqueue_put_scalars(h->b.sc, sc, h->stream);
+    CUDA_OR_FAIL(cudaGetLastError());
     CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
     return PIBM_OK;
 }
@@ -606,14 +638,21 @@ int pibm_get_particles(pibm_handle *h, double *pres, double *visc, double *force
     if (!h) return fail(PIBM_ERR_ARG, "null handle");
     const size_t n = (size_t)h->S.nbody * 3;
     if (n == 0) return PIBM_OK;
-    if (pres) CUDA_OR_FAIL(cudaMemcpyAsync(pres, h->b.pres, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    if (visc) CUDA_OR_FAIL(cudaMemcpyAsync(visc, h->b.visc, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    if (force) CUDA_OR_FAIL(cudaMemcpyAsync(force, h->b.force, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    if (!h->hpart) CUDA_OR_FAIL(cudaMallocHost(&h->hpart, 6 * n * sizeof(double)));
+    double *st = h->hpart;
+    if (pres || visc || force) CUDA_OR_FAIL(cudaMemcpyAsync(st, h->b.pres, 4 * n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     if (h->g.moving) {   // the positions and velocities the DEM has advanced
-        if (xc) CUDA_OR_FAIL(cudaMemcpyAsync(xc, h->g.xc, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-        if (vel) CUDA_OR_FAIL(cudaMemcpyAsync(vel, h->g.vel, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        if (xc) CUDA_OR_FAIL(cudaMemcpyAsync(st + 4 * n, h->g.xc, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        if (vel) CUDA_OR_FAIL(cudaMemcpyAsync(st + 5 * n, h->g.vel, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     }
     CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
+    if (pres) std::memcpy(pres, st, n * sizeof(double));
+    if (visc) std::memcpy(visc, st + n, n * sizeof(double));
+    if (force) std::memcpy(force, st + 3 * n, n * sizeof(double));
+    if (h->g.moving) {
+        if (xc) std::memcpy(xc, st + 4 * n, n * sizeof(double));
+        if (vel) std::memcpy(vel, st + 5 * n, n * sizeof(double));
+    }
     if (!h->g.moving) {
         if (xc) std::memcpy(xc, h->S.xc.data(), n * sizeof(double));
         if (vel) std::memcpy(vel, h->S.vel.data(), n * sizeof(double));
@@ -963,34 +1002,28 @@ int pibm_get_contacts(pibm_handle *h, int32_t maxn, int32_t *neigh, int32_t *pn,
     return PIBM_OK;
 }
 
+// Planes 1..nx of a spectral scalar in the reference layout f(nx+1, my2, mz), x
+// fastest, plane nx+1 = plane 1 / *ratio (a device scalar), copied to the host.
+static int copy_scalar_field(pibm_handle *h, const double2 *d, const double *ratio, double *f) {
+    const Geo &g = h->g;
+    const size_t nf = (size_t)(g.nx + 1) * g.PS;
+    if (!h->stage) CUDA_OR_FAIL(h->alloc(&h->stage, 3 * nf));
+    enqueue_d2f(d, h->stage, g.nx, g.nx + 1, g.PS, 1, h->stream, ratio);
+    CUDA_OR_FAIL(cudaGetLastError());
+    CUDA_OR_FAIL(cudaMemcpyAsync(f, h->stage, nf * sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
+    return PIBM_OK;
+}
+
 int pibm_get_scalar(pibm_handle *h, double *phif, double *flux_body, double *ratios) {
     if (!h) return fail(PIBM_ERR_ARG, "null handle");
     if (!h->g.scal) return fail(PIBM_ERR_ARG, "this run has no scalar (ISCALON = 0)");
     const Geo &g = h->g;
+    int rc;
+    if (phif && (rc = copy_scalar_field(h, h->b.phif, &h->b.sc->heat_ratio, phif))) return rc;
+    if (flux_body && g.nbody)
+        CUDA_OR_FAIL(cudaMemcpyAsync(flux_body, h->b.flux_body, (size_t)g.nbody * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     Scal sc;
-    CUDA_OR_FAIL(cudaMemcpyAsync(&sc, h->b.sc, sizeof(sc), cudaMemcpyDeviceToHost, h->stream));
-    std::vector<double2> dev((size_t)g.nx * g.PS);
-    if (phif) CUDA_OR_FAIL(cudaMemcpyAsync(dev.data(), h->b.phif, dev.size() * sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
-    std::vector<double> fb((size_t)g.nbody);
-    if (flux_body && g.nbody) CUDA_OR_FAIL(cudaMemcpyAsync(fb.data(), h->b.flux_body, fb.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
-    if (phif) {
-        // reference layout phif(nx+1, my2, mz), x fastest; plane nx+1 = phif(1)/heat_ratio
-        const size_t nxf = (size_t)g.nx + 1;
-        for (int k = 0; k < g.mz; ++k)
-            for (int j = 0; j < g.my2; ++j) {
-                const size_t e = (size_t)k * g.my2 + j;
-                for (int i = 0; i < g.nx; ++i) {
-                    const double2 v = dev[(size_t)i * g.PS + e];
-                    phif[2 * (i + nxf * e)] = v.x;
-                    phif[2 * (i + nxf * e) + 1] = v.y;
-                }
-                const double2 v = dev[e];
-                phif[2 * (g.nx + nxf * e)] = v.x / sc.heat_ratio;
-                phif[2 * (g.nx + nxf * e) + 1] = v.y / sc.heat_ratio;
-            }
-    }
-    if (flux_body) for (int m = 0; m < g.nbody; ++m) flux_body[m] = fb[m];
+    if ((rc = read_scalars(h, &sc))) return rc;
     if (ratios) { ratios[0] = sc.heat_ratio; ratios[1] = sc.heat_ratio_old; ratios[2] = sc.nusselt; }
     return PIBM_OK;
 }
@@ -1011,24 +1044,9 @@ int pibm_set_desired_means(pibm_handle *h, const double *usmean_des, const doubl
 int pibm_get_scalar_nl(pibm_handle *h, double *nlphif) {
     if (!h || !nlphif) return fail(PIBM_ERR_ARG, "null argument");
     if (!h->g.scal) return fail(PIBM_ERR_ARG, "this run has no scalar (ISCALON = 0)");
-    const Geo &g = h->g;
-    Scal sc;
-    CUDA_OR_FAIL(cudaMemcpyAsync(&sc, h->b.sc, sizeof(sc), cudaMemcpyDeviceToHost, h->stream));
-    std::vector<double2> dev((size_t)g.nx * g.PS);
-    CUDA_OR_FAIL(cudaMemcpyAsync(dev.data(), h->b.nls[h->cur ^ 1], dev.size() * sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
+    const int rc = copy_scalar_field(h, h->b.nls[h->cur ^ 1], &h->b.sc->heat_ratio_old, nlphif);
+    if (rc) return rc;
     CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
-    const size_t nxf = (size_t)g.nx + 1;
-    for (int k = 0; k < g.mz; ++k)
-        for (int j = 0; j < g.my2; ++j) {
-            const size_t e = (size_t)k * g.my2 + j;
-            for (int i = 0; i < g.nx; ++i) {
-                const double2 v = dev[(size_t)i * g.PS + e];
-                nlphif[2 * (i + nxf * e)] = v.x;
-                nlphif[2 * (i + nxf * e) + 1] = v.y;
-            }
-            nlphif[2 * (g.nx + nxf * e)] = dev[e].x / sc.heat_ratio_old;
-            nlphif[2 * (g.nx + nxf * e) + 1] = dev[e].y / sc.heat_ratio_old;
-        }
     return PIBM_OK;
 }
 
@@ -1449,7 +1467,10 @@ static int batch_enqueue(pibm_batch *bt, int nsteps) {
 static int batch_reports(pibm_batch *bt) {
     CUDA_OR_FAIL(cudaStreamSynchronize(bt->stream));
     int rc = PIBM_OK;
-    for (auto *h : bt->members) { int r = fill_report(h, nullptr); if (r && !rc) rc = r; }
+    for (auto *h : bt->members) CUDA_OR_FAIL(cudaMemcpyAsync(h->hsc, h->b.sc, sizeof(Scal), cudaMemcpyDeviceToHost, bt->stream));
+    CUDA_OR_FAIL(cudaStreamSynchronize(bt->stream));
+    for (auto *h : bt->members)
+        if (h->hsc->status && !rc) rc = fail(h->hsc->status, "step reported a solver stop condition");
     return rc;
 }
 

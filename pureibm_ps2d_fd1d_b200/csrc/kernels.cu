@@ -1199,14 +1199,21 @@ __global__ void k_f2d(const double2 *__restrict__ f, double2 *__restrict__ d, in
         if (e < PS && i < nx) dc[(size_t)i * PS + e] = tile[threadIdx.x][r];
     }
 }
-__global__ void k_d2f(const double2 *__restrict__ d, double2 *__restrict__ f, int nx, int nxf, int PS, int ncomp) {
+// Plane nxf > nx is the image of plane 1, divided by *ratio when given (the
+// scalar's image plane).
+__global__ void k_d2f(const double2 *__restrict__ d, double2 *__restrict__ f, int nx, int nxf, int PS, int ncomp,
+                      const double *ratio) {
     __shared__ double2 tile[32][33];
     const int comp = blockIdx.z;
     const int i0 = blockIdx.x * 32, e0 = blockIdx.y * 32;
     const double2 *dc = d + (size_t)comp * PS * nx;
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
         const int i = i0 + r, e = e0 + threadIdx.x;
-        if (e < PS && i < nxf) tile[r][threadIdx.x] = dc[(size_t)(i == nx ? 0 : i) * PS + e];
+        if (e < PS && i < nxf) {
+            double2 v = dc[(size_t)(i == nx ? 0 : i) * PS + e];
+            if (ratio && i == nx) { const double h = *ratio; v = make_double2(v.x / h, v.y / h); }
+            tile[r][threadIdx.x] = v;
+        }
     }
     __syncthreads();
     double2 *fc = f + (size_t)comp * PS * nxf;
@@ -1214,6 +1221,13 @@ __global__ void k_d2f(const double2 *__restrict__ d, double2 *__restrict__ f, in
         const int e = e0 + r, i = i0 + threadIdx.x;
         if (e < PS && i < nxf) fc[(size_t)e * nxf + i] = tile[threadIdx.x][r];
     }
+}
+// The scalars a host sets with its state (pibm_set_state), the rest kept.
+__global__ void k_put_scalars(Scal *sc, const Scal v) {
+    if (threadIdx.x != 0) return;
+    for (int d = 0; d < 3; ++d) { sc->umean[d] = v.umean[d]; sc->mpg[d] = v.mpg[d]; sc->ufmean[d] = v.ufmean[d]; }
+    sc->t = v.t; sc->dt = v.dt; sc->cf = v.cf;
+    sc->status = 0;
 }
 
 // Standalone batched plane transforms (pibm_ff2rc / pibm_ff2cr) on natural
@@ -1405,10 +1419,6 @@ void enqueue_batch_step(int n, const MemberSet &ms, const BatchShape &bs, cudaSt
         case 128: enqueue_batch_step_t<128>(ms, bs, s, side, fork, join); break;
         case 256: enqueue_batch_step_t<256>(ms, bs, s, side, fork, join); break;
     }
-}
-// Kernels one fused batch step launches.
-int batch_kernels_per_step(const BatchShape &bs) {
-    return 6 + (bs.max_nbody > 0 ? 3 + (bs.max_nbk > 0 ? 2 + (bs.max_spn > 0 ? 1 : 0) : 0) : 0);
 }
 
 // ============================================================================
@@ -1771,9 +1781,10 @@ void enqueue_f2d(const double2 *f, double2 *d, int nx, int nxf, int PS, int ncom
     dim3 grid((nx + 31) / 32, (PS + 31) / 32, ncomp);
     k_f2d<<<grid, dim3(32, 8), 0, s>>>(f, d, nx, nxf, PS, ncomp);
 }
-void enqueue_d2f(const double2 *d, double2 *f, int nx, int nxf, int PS, int ncomp, cudaStream_t s) {
+void enqueue_d2f(const double2 *d, double2 *f, int nx, int nxf, int PS, int ncomp, cudaStream_t s, const double *ratio) {
     dim3 grid((nxf + 31) / 32, (PS + 31) / 32, ncomp);
-    k_d2f<<<grid, dim3(32, 8), 0, s>>>(d, f, nx, nxf, PS, ncomp);
+    k_d2f<<<grid, dim3(32, 8), 0, s>>>(d, f, nx, nxf, PS, ncomp, ratio);
 }
+void enqueue_put_scalars(Scal *sc, const Scal &v, cudaStream_t s) { k_put_scalars<<<1, 32, 0, s>>>(sc, v); }
 
 }  // namespace pibm
