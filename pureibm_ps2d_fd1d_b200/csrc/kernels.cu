@@ -885,6 +885,13 @@ __global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) k_ff(Geo g, const doubl
 // Tiles live in shared memory as [line][i]; global loads and stores run over
 // consecutive lines (contiguous in the [i][k][j] layout).
 // ============================================================================
+// Threads per tile: a warp per line for the solves; at 256, where a tile's 93 KB
+// leave two blocks per SM, a second warp per line for the passes over the
+// tile, which wait on their loads (k_lines 1209 -> 1005 us).
+template <int NX, int LT> __host__ __device__ constexpr int lines_threads() { return LT * 32 * (NX >= 256 && LT == 4 ? 2 : 1); }
+// Blocks per SM the register budget is sized for (the batch's indexed
+// parameter loads would raise the count).
+template <int NX, int LT> __host__ __device__ constexpr int lines_minb() { return NX <= 128 ? (LT == 4 ? 4 : 2) : (LT == 4 ? 2 : 1); }
 template <int NX, int LT>
 __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, double2 *__restrict__ p,
                                                    const double2 *__restrict__ nl, const double2 *__restrict__ onl,
@@ -949,7 +956,7 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
     }
     __syncthreads();
     const int qw = q0 + w;
-    const bool wact = qw < PS;
+    const bool wact = w < LT && qw < PS;   // warp w < LT solves line w
     const double w2w = wact ? g.w2[qw] : 0.0;
     const LineCoef kw = line_coef(dt, vis, c1, c2, dx2, w2w);   // line qw's coefficients
     {
@@ -966,7 +973,7 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
     }
     __syncthreads();
     // ---------------- ustep per component (usteptime.F90:73-470) ----------------
-    constexpr int EPT = (LT * NX) / (LT * 32);   // tile elements per thread
+    constexpr int T = lines_threads<NX, LT>(), EPT = (LT * NX) / T;   // tile elements per thread
     const Circ<R> ku = circ_factor<R>(kw.ua, kw.ub);
     for (int n = 0; n < 3; ++n) {
         // stage u_n of the tile, then form every right-hand side from the staged
@@ -979,7 +986,7 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
         double2 rr[EPT];
 #pragma unroll
         for (int k = 0; k < EPT; ++k) {
-            const int t = threadIdx.x + k * LT * 32;
+            const int t = threadIdx.x + k * T;
             const int line = t % LT, i = t / LT, q = q0 + line;
             if (q >= PS) continue;
             const LineCoef kq = line_coef(dt, vis, c1, c2, dx2, g.w2[q]);
@@ -990,7 +997,7 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < EPT; ++k) {
-            const int t = threadIdx.x + k * LT * 32;
+            const int t = threadIdx.x + k * T;
             const int line = t % LT, i = t / LT, q = q0 + line;
             if (q < PS) RHS[line * NP + row_slot(i)] = rr[k];
         }
@@ -1057,7 +1064,7 @@ __device__ __forceinline__ void b_lines(const Geo &g, double2 *__restrict__ u, d
     }
 }
 template <int NX, int LT>
-__global__ void __launch_bounds__(LT * 32) k_lines(Geo g, double2 *__restrict__ u, double2 *__restrict__ p,
+__global__ void __launch_bounds__(lines_threads<NX, LT>(), lines_minb<NX, LT>()) k_lines(Geo g, double2 *__restrict__ u, double2 *__restrict__ p,
                                                    const double2 *__restrict__ nl, const double2 *__restrict__ onl,
                                                    const double2 *__restrict__ ff, Scal *__restrict__ sc) { b_lines<NX, LT>(g, u, p, nl, onl, ff, sc); }
 
@@ -1159,7 +1166,7 @@ static void launch_lines(const Geo &g, DevBufs &b, double2 *u, double2 *p, int c
             }
         }
     }
-    if (lt == 4) k_lines<N, 4><<<(g.PS + 3) / 4, 4 * 32, lines_smem<N>(4), s>>>(g, u, p, b.nl[cur], b.nl[old], b.ff, sc);
+    if (lt == 4) k_lines<N, 4><<<(g.PS + 3) / 4, lines_threads<N, 4>(), lines_smem<N>(4), s>>>(g, u, p, b.nl[cur], b.nl[old], b.ff, sc);
     else k_lines<N, 8><<<(g.PS + 7) / 8, 8 * 32, lines_smem<N>(8), s>>>(g, u, p, b.nl[cur], b.nl[old], b.ff, sc);
 }
 
@@ -1355,11 +1362,8 @@ __global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) kb_ff(const __grid_cons
     if (m.g.nbody == 0) return;
     b_ff<N>(m.g, m.b.fr, m.b.ff, m.b.sc);
 }
-// CTAs per SM of the single-run x-line kernels at their register counts,
-// kept as a bound here (the indexed parameter loads would raise the count).
-template <int N, int LT> constexpr int kb_lines_minb() { return N <= 128 ? (LT == 4 ? 4 : 2) : (LT == 4 ? 2 : 1); }
 template <int N, int LT>
-__global__ void __launch_bounds__(LT * 32, kb_lines_minb<N, LT>()) kb_lines(const __grid_constant__ MemberSet ms) {
+__global__ void __launch_bounds__(lines_threads<N, LT>(), lines_minb<N, LT>()) kb_lines(const __grid_constant__ MemberSet ms) {
     const Member &m = ms.m[blockIdx.z];
     b_lines<N, LT>(m.g, m.b.u, m.b.p, m.b.nl[m.cur], m.b.nl[m.cur ^ 1], m.b.ff, m.b.sc);
 }
@@ -1405,7 +1409,7 @@ static void enqueue_batch_step_t(const MemberSet &ms, const BatchShape &bs, cuda
         launch_planes_z<RL<N>>(kb_ff<N>, N, 3, nz, s, ms);
     }
     const int PS = (N / 2 + 1) * N;
-    if (bs.lines_lt == 4) kb_lines<N, 4><<<dim3((PS + 3) / 4, 1, nz), 4 * 32, lines_smem<N>(4), s>>>(ms);
+    if (bs.lines_lt == 4) kb_lines<N, 4><<<dim3((PS + 3) / 4, 1, nz), lines_threads<N, 4>(), lines_smem<N>(4), s>>>(ms);
     else kb_lines<N, 8><<<dim3((PS + 7) / 8, 1, nz), 8 * 32, lines_smem<N>(8), s>>>(ms);
     kb_scal_d<<<dim3(1, 1, nz), 32, 0, s>>>(ms);
 }
@@ -1504,7 +1508,11 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
     // kernels then start with the x flux and fill the GPU, and the flow's short
     // side kernels measured slower queued beside them.
     const bool fork = ss && !ev && !kev;
-    const bool scal_first = g.scal && !g.moving;
+    // At 256 the scalar step follows on the main stream: its plane kernels and
+    // the flow's, clusters of 8 CTAs each, then only take each other's SMs
+    // (moving suspension with scalar: 13.9 ms per step forked, 12.7 in turn).
+    constexpr bool scal_beside = N <= 128;
+    const bool scal_first = g.scal && !g.moving && scal_beside;
     mark(0);
     kb(PIBM_K_A0);
     launch_planes_pdl<PL<N>>(k_a0<N>, g.nx, 10, s, g, (const double2 *)b.u, (const double2 *)b.p, b.ubcp, b.pbcp, b.omega, b.pgr, b.sc, b.part);
@@ -1553,7 +1561,7 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
         }
         if (g.moving) {
             enqueue_moving(g, b.mov, b.sc, b.pres, b.visc, s);
-            if (fork && g.scal) {   // the scalar step needs the new geometry
+            if (fork && g.scal && scal_beside) {   // the scalar step needs the new geometry
                 cudaEventRecord(ss->geo_done, s);
                 cudaStreamWaitEvent(ss->scal, ss->geo_done, 0);
                 enqueue_scalar(g, b, cur, ss->scal);
@@ -1605,7 +1613,7 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
     ke(PIBM_K_SCAL_D);
     mark(6);
     if (g.scal) {
-        if (fork) cudaStreamWaitEvent(s, ss->scal_done, 0);
+        if (fork && scal_beside) cudaStreamWaitEvent(s, ss->scal_done, 0);
         else enqueue_scalar(g, b, cur, s);
     }
     mark(7);
