@@ -301,6 +301,7 @@ int pibm_create(const pibm_params *prm, const pibm_particles *parts, pibm_handle
         sp_node_p[q] = i * g.RS + roff[e];
     }
     DevBufs &b = h->b;
+    const bool sweeps = S.my >= kSweepMin;
     bool ok = guard(h->upload(&g.tw, tw), "tw") && guard(h->upload(&g.ky, S.ky), "ky") && guard(h->upload(&g.kz, S.kz), "kz") &&
               guard(h->upload(&g.w2, S.w2), "w2") && guard(h->upload(&g.fluid, fluid_p), "mask") &&
               guard(h->upload(&g.xc, S.xc), "xc") && guard(h->upload(&g.vel, S.vel), "vel") &&
@@ -310,17 +311,23 @@ int pibm_create(const pibm_params *prm, const pibm_particles *parts, pibm_handle
               guard(h->upload(&g.sp_ptr, S.sp_ptr), "sp_ptr") && guard(h->upload(&g.sp_ent, S.sp_ent), "sp_ent") &&
               guard(h->alloc(&b.u, 3 * NC), "u") && guard(h->alloc(&b.p, NC), "p") &&
               guard(h->alloc(&b.nl[0], 3 * NC), "nl0") && guard(h->alloc(&b.nl[1], 3 * NC), "nl1") &&
-              guard(h->alloc(&b.ff, 3 * NC), "ff") && guard(h->alloc(&b.ubcp, 3 * NR), "ubcp") &&
-              guard(h->alloc(&b.pbcp, NR), "pbcp") && guard(h->alloc(&b.Q, 3 * NR), "Q") && guard(h->alloc(&b.Dx, 3 * NR), "Dx") &&
+              (sweeps ? guard(h->alloc(&b.wz, 11 * NC), "Dx, Q, ff and sweeps")
+                      : guard(h->alloc(&b.Q, 3 * NR), "Q") && guard(h->alloc(&b.Dx, 3 * NR), "Dx")) &&
+              ((sweeps && S.nbody > 0) || guard(h->alloc(&b.ff, 3 * NC), "ff")) &&
+              guard(h->alloc(&b.ubcp, 3 * NR), "ubcp") && guard(h->alloc(&b.pbcp, NR), "pbcp") &&
               guard(h->alloc(&b.omega, 3 * NR), "omega") && guard(h->alloc(&b.pgr, 3 * NR), "pgr") &&
               (S.nbody == 0 || guard(h->alloc(&b.fr, 3 * NR), "fr")) &&
-              guard(h->alloc(&b.part, (size_t)g.nx * 8 * 12), "part") &&
+              guard(h->alloc(&b.part, (size_t)g.nx * 16 * 12), "part") &&
               guard(h->alloc(&b.pres, 12 * (size_t)S.nbody), "particle forces") &&
               guard(h->alloc(&b.rec, 6 * (size_t)g.npts), "rec") && guard(h->alloc(&b.rz, 3 * (size_t)g.npts), "rz") &&
               guard(h->alloc(&b.dpart, 6 * 8 * (size_t)S.nbody), "dpart") &&
               guard(h->alloc(&b.blockpart, 6 * (size_t)((g.npts + 255) / 256 + 1)), "blockpart") &&
               guard(h->alloc(&b.sc, 1), "scalars");
     if (!ok) { delete h; return rc; }
+    if (sweeps) {   // FlowBufs::wz
+        b.Dx = (double *)b.wz; b.Q = (double *)(b.wz + 3 * NC);
+        if (S.nbody > 0) b.ff = b.wz + 6 * NC;   // without spheres ff stays zero
+    }
     // pres, visc, ptot and force are one block: one copy reads them back
     b.visc = b.pres + 3 * (size_t)S.nbody; b.ptot = b.visc + 3 * (size_t)S.nbody; b.force = b.ptot + 3 * (size_t)S.nbody;
     if (S.scal) {

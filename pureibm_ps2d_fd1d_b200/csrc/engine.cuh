@@ -5,6 +5,8 @@
 
 namespace pibm {
 
+constexpr int kSweepMin = 256;   // grids from this size on transform by sweeps (sweep.cuh)
+
 // Per-run constants passed by value to every kernel.
 struct Geo {
     int nx, my, mz, my2;
@@ -106,6 +108,12 @@ struct Mov {
 // The flow step's buffers (what the step kernels read and write).
 struct FlowBufs {
     double2 *u, *p, *nl[2], *ff;
+    // 256^3: Dx, Q, ff (3 slots of a spectral field each) and 2 slots more,
+    // which also take the (z, ky) planes of the sweeps while they are dead: the
+    // 7 fields (before Dx and Q are formed) slots 0-6, the 8 products (Dx still
+    // read) slots 3-10, Q's planes slots 6-8, the forcing's (Dx dead) slots 0-2.
+    // fr keeps its own: its unforced nodes stay zero from step to step.
+    double2 *wz;
     double *ubcp, *pbcp, *Q, *omega, *pgr, *fr, *Dx;
     double *part, *pres, *visc, *ptot, *force, *rec, *rz, *dpart, *blockpart;
     Scal *sc;

@@ -9,13 +9,15 @@
 // across consecutive lines).  The periodic image plane nx+1 of the reference
 // is never stored; x indices wrap instead.
 //
-// Step pipeline (reference routines in brackets):
+// Step pipeline (reference routines in brackets; at 256^3 k_a0, k_nl and k_ff
+// are the column and row sweeps of sweep.cuh):
 //   k_a0      10 c2r per plane: ubcp (+umean), pbcp, omega, grad p (without mpg);
 //             fluid/solid means and max|u|       [compute_new_timestep, calc_pressure,
 //                                                   compute_omega, calc_pgrad]
 //   k_scal_a  CFL dt, t, cf (soft start), ufmean, mean slip   [compute_new_timestep]
+//   k_flux    x-flux differences                    [form_nl]
 //   k_nl      products + x flux, 9 r2c -> nl; 3 c2r -> Q = -c3 nl - c4 onl - c12 diffn
-//                                                  [form_nl, nonlinear, calc_visc]
+//                                                  [nonlinear, calc_visc]
 //   k_drag    per-sphere surface quadrature of p and omega     [calc_pres_visc_drag]
 //   k_scal_b  pres/visc totals, mpg, per-sphere force, drag diagnostics   [compute_mpg_at_n, bcset]
 //   k_rev     reversal-point force per active point            [calc_inner_reversal_forcing]
@@ -32,6 +34,7 @@
 #include "step_common.cuh"
 #include "line_solve.cuh"
 #include "lines_pipe.cuh"
+#include "sweep.cuh"
 #include "../../include/pibm.h"
 
 namespace pibm {
@@ -1295,6 +1298,70 @@ __global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) k_ff2rc(Geo g, const do
     });
 }
 
+// The column and row sweeps of the larger grids (sweep.cuh).
+template <int N> constexpr bool use_sweeps() { return N >= kSweepMin; }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 5) k_cz(Geo g, const double2 *__restrict__ u, const double2 *__restrict__ p, double2 *__restrict__ zf) { b_cz<N>(g, u, p, zf); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) k_ry(Geo g, const double2 *__restrict__ zf, double *__restrict__ ubcp, double *__restrict__ pbcp, double *__restrict__ omega,
+                                                                       double *__restrict__ pgr, Scal *__restrict__ sc, double *__restrict__ part) { b_ry<N>(g, zf, ubcp, pbcp, omega, pgr, sc, part); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) k_rp(Geo g, const double *__restrict__ ubcp, const double *__restrict__ Dx, double2 *__restrict__ pz, Scal *__restrict__ sc) { b_rp<N>(g, ubcp, Dx, pz, sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 4) k_cn(Geo g, const double2 *__restrict__ pz, double2 *nl_new) { b_cn<N>(g, pz, nl_new); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 4) k_cq(Geo g, const double2 *__restrict__ nl, const double2 *__restrict__ u, const double2 *__restrict__ onl,
+                                                                       double2 *__restrict__ qz) { b_cq<N>(g, nl, u, onl, qz); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) k_rq(Geo g, const double2 *__restrict__ qz, double *__restrict__ Q, Scal *__restrict__ sc) { b_rq<N>(g, qz, Q, sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) k_rf(Geo g, const double *__restrict__ fr, double2 *__restrict__ fz, Scal *__restrict__ sc) { b_rf<N>(g, fr, fz, sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 5) k_cf(Geo g, const double2 *__restrict__ fz, double2 *__restrict__ ff) { b_cf<N>(g, fz, ff); }
+// A launch that may start its prologue while the previous kernel of the stream drains.
+template <typename... KArgs, typename... Args>
+static void launch_pdl(void (*k)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, args...);
+}
+// The step's plane transforms: fields to real space, nonlinear term and Q, forcing.
+// Slots of the sweeps' (z, ky) planes in FlowBufs::wz.
+template <int N> __host__ __device__ __forceinline__ double2 *wz_products(double2 *wz) { return wz + 3 * (size_t)N * Sweep<N>::PS; }
+template <int N> __host__ __device__ __forceinline__ double2 *wz_q(double2 *wz) { return wz + 6 * (size_t)N * Sweep<N>::PS; }
+template <int N> static void enqueue_a0(const Geo &g, DevBufs &b, cudaStream_t s) {
+    if constexpr (use_sweeps<N>()) {
+        using W = Sweep<N>;
+        launch_pdl(k_cz<N>, dim3(7, W::GC), W::CT, W::CSM, s, g, (const double2 *)b.u, (const double2 *)b.p, b.wz);
+        launch_pdl(k_ry<N>, dim3(10, N * W::RB), W::RT, W::RSM, s, g, (const double2 *)b.wz, b.ubcp, b.pbcp, b.omega, b.pgr, b.sc, b.part);
+    } else {
+        launch_planes_pdl<PL<N>>(k_a0<N>, g.nx, 10, s, g, (const double2 *)b.u, (const double2 *)b.p, b.ubcp, b.pbcp, b.omega, b.pgr, b.sc, b.part);
+    }
+}
+template <int N> static void enqueue_nl(const Geo &g, DevBufs &b, int cur, cudaStream_t s) {
+    const int old = cur ^ 1;
+    if constexpr (use_sweeps<N>()) {
+        using W = Sweep<N>;
+        double2 *pz = wz_products<N>(b.wz), *qz = wz_q<N>(b.wz);
+        launch_pdl(k_rp<N>, dim3(8, N * W::RB), W::RT, W::RSM, s, g, (const double *)b.ubcp, (const double *)b.Dx, pz, b.sc);
+        launch_pdl(k_cn<N>, dim3(3, W::GC), W::CT, W::CSM, s, g, (const double2 *)pz, b.nl[cur]);
+        launch_pdl(k_cq<N>, dim3(3, W::GC), W::CT, W::CSM, s, g, (const double2 *)b.nl[cur], (const double2 *)b.u, (const double2 *)b.nl[old], qz);
+        launch_pdl(k_rq<N>, dim3(3, N * W::RB), W::RT, W::RSM, s, g, (const double2 *)qz, b.Q, b.sc);
+    } else {
+        launch_planes_pdl<NL<N>>(k_nl<N>, g.nx, 3, s, g, (const double *)b.ubcp, (const double *)b.Dx, (const double2 *)b.u,
+                                 (const double2 *)b.nl[old], b.nl[cur], b.Q, b.sc);
+    }
+}
+template <int N> static void enqueue_ff(const Geo &g, DevBufs &b, Scal *sc, cudaStream_t s) {
+    if constexpr (use_sweeps<N>()) {
+        using W = Sweep<N>;
+        launch_pdl(k_rf<N>, dim3(3, N * W::RB), W::RT, W::RSM, s, g, (const double *)b.fr, b.wz, sc);
+        launch_pdl(k_cf<N>, dim3(3, W::GC), W::CT, W::CSM, s, g, (const double2 *)b.wz, b.ff);
+    } else {
+        launch_planes_pdl<RL<N>>(k_ff<N>, g.nx, 3, s, g, (const double *)b.fr, b.ff, sc);
+    }
+}
+
 // ============================================================================
 // Fused batch step: the kernels of one time step for every run of a batch
 // that has the same grid size, one launch per kernel, the runs along
@@ -1319,6 +1386,17 @@ __global__ void __launch_bounds__(256, 4) kb_flux(const __grid_constant__ Member
     const Member &m = ms.m[blockIdx.z];
     b_flux<N>(m.g, m.b.ubcp, m.b.Dx, m.b.sc);
 }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 5) kb_cz(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_cz<N>(m.g, m.b.u, m.b.p, m.b.wz); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) kb_ry(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_ry<N>(m.g, m.b.wz, m.b.ubcp, m.b.pbcp, m.b.omega, m.b.pgr, m.b.sc, m.b.part); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) kb_rp(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_rp<N>(m.g, m.b.ubcp, m.b.Dx, wz_products<N>(m.b.wz), m.b.sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 4) kb_cn(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_cn<N>(m.g, wz_products<N>(m.b.wz), m.b.nl[m.cur]); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 4) kb_cq(const __grid_constant__ MemberSet ms) {
+    const Member &m = ms.m[blockIdx.z];
+    b_cq<N>(m.g, m.b.nl[m.cur], m.b.u, m.b.nl[m.cur ^ 1], wz_q<N>(m.b.wz));
+}
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) kb_rq(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_rq<N>(m.g, wz_q<N>(m.b.wz), m.b.Q, m.b.sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) kb_rf(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; if (m.g.nbody == 0) return; b_rf<N>(m.g, m.b.fr, m.b.wz, m.b.sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 5) kb_cf(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; if (m.g.nbody == 0) return; b_cf<N>(m.g, m.b.wz, m.b.ff); }
 template <int N>
 __global__ void __launch_bounds__(NL<N>::T, NL<N>::MINB) kb_nl(const __grid_constant__ MemberSet ms) {
     const Member &m = ms.m[blockIdx.z];
@@ -1379,7 +1457,12 @@ template <int N>
 static void enqueue_batch_step_t(const MemberSet &ms, const BatchShape &bs, cudaStream_t s, cudaStream_t side,
                                  cudaEvent_t fork, cudaEvent_t join) {
     const int nz = bs.nz;
-    launch_planes_z<PL<N>>(kb_a0<N>, N, 10, nz, s, ms);
+    if constexpr (use_sweeps<N>()) {
+        kb_cz<N><<<dim3(7, Sweep<N>::GC, nz), Sweep<N>::CT, Sweep<N>::CSM, s>>>(ms);
+        kb_ry<N><<<dim3(10, N * Sweep<N>::RB, nz), Sweep<N>::RT, Sweep<N>::RSM, s>>>(ms);
+    } else {
+        launch_planes_z<PL<N>>(kb_a0<N>, N, 10, nz, s, ms);
+    }
     const bool spheres = bs.max_nbody > 0;
     cudaEventRecord(fork, s);
     cudaStreamWaitEvent(side, fork, 0);
@@ -1390,7 +1473,14 @@ static void enqueue_batch_step_t(const MemberSet &ms, const BatchShape &bs, cuda
     }
     cudaEventRecord(join, side);
     kb_flux<N><<<dim3((RP<N>::RSP * (N / bs.flux_seg) + 255) / 256, 1, nz), 256, 0, s>>>(ms);
-    launch_planes_z<NL<N>>(kb_nl<N>, N, 3, nz, s, ms);
+    if constexpr (use_sweeps<N>()) {
+        kb_rp<N><<<dim3(8, N * Sweep<N>::RB, nz), Sweep<N>::RT, Sweep<N>::RSM, s>>>(ms);
+        kb_cn<N><<<dim3(3, Sweep<N>::GC, nz), Sweep<N>::CT, Sweep<N>::CSM, s>>>(ms);
+        kb_cq<N><<<dim3(3, Sweep<N>::GC, nz), Sweep<N>::CT, Sweep<N>::CSM, s>>>(ms);
+        kb_rq<N><<<dim3(3, N * Sweep<N>::RB, nz), Sweep<N>::RT, Sweep<N>::RSM, s>>>(ms);
+    } else {
+        launch_planes_z<NL<N>>(kb_nl<N>, N, 3, nz, s, ms);
+    }
     cudaStreamWaitEvent(s, join, 0);
     if (spheres) {
         if (bs.max_nbk > 0) {
@@ -1406,7 +1496,12 @@ static void enqueue_batch_step_t(const MemberSet &ms, const BatchShape &bs, cuda
             }
             cudaStreamWaitEvent(s, join, 0);
         }
-        launch_planes_z<RL<N>>(kb_ff<N>, N, 3, nz, s, ms);
+        if constexpr (use_sweeps<N>()) {
+            kb_rf<N><<<dim3(3, N * Sweep<N>::RB, nz), Sweep<N>::RT, Sweep<N>::RSM, s>>>(ms);
+            kb_cf<N><<<dim3(3, Sweep<N>::GC, nz), Sweep<N>::CT, Sweep<N>::CSM, s>>>(ms);
+        } else {
+            launch_planes_z<RL<N>>(kb_ff<N>, N, 3, nz, s, ms);
+        }
     }
     const int PS = (N / 2 + 1) * N;
     if (bs.lines_lt == 4) kb_lines<N, 4><<<dim3((PS + 3) / 4, 1, nz), lines_threads<N, 4>(), lines_smem<N>(4), s>>>(ms);
@@ -1432,18 +1527,20 @@ template <int N>
 static cudaError_t set_attrs() {
     const int maxs = (int)PL<N>::SMEM;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(k_a0<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_nl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NL<N>::SMEM)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_ff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
+    if constexpr (!use_sweeps<N>()) {
+        if ((e = cudaFuncSetAttribute(k_a0<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(k_nl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NL<N>::SMEM)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(k_ff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(kb_a0<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(kb_nl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NL<N>::SMEM)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(kb_ff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
+    }
     if ((e = cudaFuncSetAttribute(k_ff2cr<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_ff2rc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_lines<N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lines_smem<N>(4))) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_lines<N, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lines_smem<N>(8))) != cudaSuccess) return e;
     if constexpr (N <= 128)
         if ((e = cudaFuncSetAttribute(k_lines_pipe<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, LPipe<N>::SMEM)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_a0<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_nl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NL<N>::SMEM)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_ff<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL<N>::SMEM)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(kb_lines<N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lines_smem<N>(4))) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(kb_lines<N, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lines_smem<N>(8))) != cudaSuccess) return e;
     return cudaSuccess;
@@ -1469,7 +1566,7 @@ int plane_ctas(int n) {
         case 64: return PL<64>::C;
         case 96: return PL<96>::C;
         case 128: return PL<128>::C;
-        case 256: return PL<256>::C;
+        case 256: return Sweep<256>::RB;
         default: return 1;
     }
 }
@@ -1495,7 +1592,6 @@ int real_offset(int n, int z, int y) {
 template <int N>
 static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cudaEvent_t *ev, const StepStreams *ss,
                            cudaEvent_t *kev) {
-    const int old = 1 - cur;
     auto mark = [&](int q) { if (ev) cudaEventRecord(ev[q], s); };
     auto kb = [&](int k) { if (kev) cudaEventRecord(kev[2 * k], s); };
     auto ke = [&](int k) { if (kev) cudaEventRecord(kev[2 * k + 1], s); };
@@ -1515,7 +1611,7 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
     const bool scal_first = g.scal && !g.moving && scal_beside;
     mark(0);
     kb(PIBM_K_A0);
-    launch_planes_pdl<PL<N>>(k_a0<N>, g.nx, 10, s, g, (const double2 *)b.u, (const double2 *)b.p, b.ubcp, b.pbcp, b.omega, b.pgr, b.sc, b.part);
+    enqueue_a0<N>(g, b, s);
     ke(PIBM_K_A0);
     if (fork) {
         if (scal_first) k_scal_a<<<1, 256, 0, s>>>(g, b.sc, b.part);
@@ -1545,8 +1641,7 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
     else k_flux<N, 4><<<fgrid, 256, 0, s>>>(g, b.ubcp, b.Dx, b.sc);
     ke(PIBM_K_FLUX);
     kb(PIBM_K_NL);
-    launch_planes_pdl<NL<N>>(k_nl<N>, g.nx, 3, s, g, (const double *)b.ubcp, (const double *)b.Dx, (const double2 *)b.u,
-                         (const double2 *)b.nl[old], b.nl[cur], b.Q, b.sc);
+    enqueue_nl<N>(g, b, cur, s);
     ke(PIBM_K_NL);
     mark(2);
     if (fork) cudaStreamWaitEvent(s, ss->drag_done, 0);
@@ -1597,7 +1692,7 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
         }
         mark(4);
         kb(PIBM_K_FF);
-        launch_planes_pdl<RL<N>>(k_ff<N>, g.nx, 3, s, g, (const double *)b.fr, b.ff, b.sc);
+        enqueue_ff<N>(g, b, b.sc, s);
         ke(PIBM_K_FF);
     } else {
         mark(3); mark(4);
@@ -1622,6 +1717,7 @@ static void enqueue_step_t(const Geo &g, DevBufs &b, int cur, cudaStream_t s, cu
 // Kernels launched per step (for launch accounting).
 int kernels_per_step(const Geo &g, const Mov &m) {
     int n = 6;   // a0, scal_a, flux, nl, lines, scal_d
+    if (g.my >= kSweepMin) n += 4 + (g.nbody > 0 ? 1 : 0);   // a0, nl and ff as sweeps: 2, 4 and 2 launches
     if (g.nbody > 0) n += 3 + (g.npts > 0 ? 2 + (g.sp_nnodes > 0 || g.moving ? 1 : 0) : 0);
     if (g.moving) n += moving_kernels_per_step(m);
     return n + scalar_kernels_per_step(g);
@@ -1735,7 +1831,7 @@ static cudaError_t autotune_lines_t(Geo &g, DevBufs &b, int cur, cudaStream_t s,
                 // the forcing transform writes only the work field ff, which the
                 // step recomputes before its line kernel; runs without
                 // particles have no forcing (fr is not allocated, ff stays zero)
-                if (g.nbody > 0 && b.fr) launch_planes<RL<N>>(k_ff<N>, g.nx, 3, s, g, (const double *)b.fr, b.ff, sc);
+                if (g.nbody > 0 && b.fr) enqueue_ff<N>(g, b, sc, s);
                 launch_lines<N>(gt, b, u, p, cur, sc, s);
             }
         };

@@ -163,6 +163,129 @@ template <int S> __device__ __forceinline__ double2 tw_get(const double2 *tw, in
     return S > 0 ? make_double2(v.x, -v.y) : v;
 }
 
+// ---- y passes over NR rows at pitch M+1 held by T threads ----
+// c2r: rows of spectral values (natural column order; ky = 0 and M both in
+// slot 0 when kPacked, else in slots 0 and M, of which the real parts count)
+// -> rows of real pairs, pair m = k1 + AY*k2 in slot BY*k1 + k2.
+template <int N, int NR, int T, bool kPacked>
+__device__ __forceinline__ void rows_c2r(double2 *buf, const double2 *tw) {
+    constexpr int AY = Plan<N>::AY, BY = Plan<N>::BY, H = BY / 2, M = N / 2, P = M + 1;
+    const int tid = threadIdx.x;
+    // real reconstruction and y over AY (slot BY*n1 + n2), twiddle w_M^{n2 k1}
+#pragma unroll
+    for (int u0 = 0; u0 < NR * H; u0 += T) {
+        const int u = u0 + tid;
+        if (NR * H % T == 0 || u < NR * H) {
+            const int g = u / NR, ca = g, cb = g == 0 ? H : BY - g;
+            double2 *row = buf + (u % NR) * P;
+            double2 a[AY], b[AY];
+#pragma unroll
+            for (int n = 0; n < AY; ++n) { a[n] = row[ca + BY * n]; b[n] = row[cb + BY * n]; }
+            if (g == 0) {   // classes 0 (with ky = 0, M and M/2) and BY/2 mirror onto themselves
+                const double xm = kPacked ? a[0].y : row[M].x;
+                a[0] = make_double2(a[0].x + xm, a[0].x - xm);
+#pragma unroll
+                for (int n = 1; n < AY / 2; ++n) c2r_pre_pair(a[n], a[AY - n], tw_get<1>(tw, BY * n));
+                a[AY / 2] = make_double2(2.0 * a[AY / 2].x, -2.0 * a[AY / 2].y);
+#pragma unroll
+                for (int n = 0; n < AY / 2; ++n) c2r_pre_pair(b[n], b[AY - 1 - n], tw_get<1>(tw, H + BY * n));
+            } else {
+#pragma unroll
+                for (int n = 0; n < AY; ++n) c2r_pre_pair(a[n], b[AY - 1 - n], tw_get<1>(tw, g + BY * n));
+            }
+            Dft<AY, 1>::run(a);
+            row[ca] = a[0];
+#pragma unroll
+            for (int k1 = 1; k1 < AY; ++k1) row[ca + BY * k1] = cmul(a[k1], tw_get<1>(tw, 2 * ca * k1));
+            Dft<AY, 1>::run(b);
+            row[cb] = b[0];
+#pragma unroll
+            for (int k1 = 1; k1 < AY; ++k1) row[cb + BY * k1] = cmul(b[k1], tw_get<1>(tw, 2 * cb * k1));
+        }
+    }
+    __syncthreads();
+    // y over BY
+#pragma unroll
+    for (int u0 = 0; u0 < NR * AY; u0 += T) {
+        const int u = u0 + tid;
+        if (NR * AY % T == 0 || u < NR * AY) {
+            double2 *base = buf + (u % NR) * P + BY * (u / NR);
+            double2 v[BY];
+#pragma unroll
+            for (int n2 = 0; n2 < BY; ++n2) v[n2] = base[n2];
+            Dft<BY, 1>::run(v);
+#pragma unroll
+            for (int k2 = 0; k2 < BY; ++k2) base[k2] = v[k2];
+        }
+    }
+    __syncthreads();
+}
+// r2c, first pass: y over BY (slot BY*n1 + n2 holds the pair n1 + AY*n2),
+// twiddle w_M^{n1 k2}.
+template <int N, int NR, int T>
+__device__ __forceinline__ void rows_r2c_1(double2 *buf, const double2 *tw) {
+    constexpr int AY = Plan<N>::AY, BY = Plan<N>::BY, P = N / 2 + 1;
+#pragma unroll
+    for (int u0 = 0; u0 < NR * AY; u0 += T) {
+        const int u = u0 + (int)threadIdx.x;
+        if (NR * AY % T == 0 || u < NR * AY) {
+            const int n1 = u / NR;
+            double2 *base = buf + (u % NR) * P + BY * n1;
+            double2 v[BY];
+#pragma unroll
+            for (int n2 = 0; n2 < BY; ++n2) v[n2] = base[n2];
+            Dft<BY, -1>::run(v);
+            base[0] = v[0];
+#pragma unroll
+            for (int k2 = 1; k2 < BY; ++k2) base[k2] = cmul(v[k2], tw_get<-1>(tw, 2 * n1 * k2));
+        }
+    }
+    __syncthreads();
+}
+// Unit u of the second pass, y over AY (column BY*k1 + k2) and the real split:
+// columns ca + BY*k (a) and cb + BY*k (b) of row u % NR; a[0] = X[0] + i X[M].
+template <int N, int NR>
+__device__ __forceinline__ void row_unit_r2c(const double2 *buf, const double2 *tw, int u, double2 (&a)[Plan<N>::AY],
+                                             double2 (&b)[Plan<N>::AY]) {
+    constexpr int AY = Plan<N>::AY, BY = Plan<N>::BY, H = BY / 2, P = N / 2 + 1;
+    const int g = u / NR, ca = g, cb = g == 0 ? H : BY - g;
+    const double2 *row = buf + (u % NR) * P;
+#pragma unroll
+    for (int n = 0; n < AY; ++n) { a[n] = row[ca + BY * n]; b[n] = row[cb + BY * n]; }
+    Dft<AY, -1>::run(a);
+    Dft<AY, -1>::run(b);
+    if (g == 0) {   // ky = 0 and M, both real, stay packed as ky = 0 + i ky = M
+        a[0] = make_double2(a[0].x + a[0].y, a[0].x - a[0].y);
+#pragma unroll
+        for (int n = 1; n < AY / 2; ++n) r2c_post_pair(a[n], a[AY - n], tw_get<-1>(tw, BY * n));
+        a[AY / 2].y = -a[AY / 2].y;
+#pragma unroll
+        for (int n = 0; n < AY / 2; ++n) r2c_post_pair(b[n], b[AY - 1 - n], tw_get<-1>(tw, H + BY * n));
+    } else {
+#pragma unroll
+        for (int n = 0; n < AY; ++n) r2c_post_pair(a[n], b[AY - 1 - n], tw_get<-1>(tw, g + BY * n));
+    }
+}
+// r2c, second pass in place; ky = 0 and M packed in slot 0, or in slots 0 and M.
+template <int N, int NR, int T, bool kPacked>
+__device__ __forceinline__ void rows_r2c_2(double2 *buf, const double2 *tw) {
+    constexpr int AY = Plan<N>::AY, BY = Plan<N>::BY, H = BY / 2, TOT = NR * H, M = N / 2, P = M + 1;
+#pragma unroll
+    for (int u0 = 0; u0 < TOT; u0 += T) {
+        const int u = u0 + (int)threadIdx.x;
+        if (TOT % T == 0 || u < TOT) {
+            double2 a[AY], b[AY];
+            row_unit_r2c<N, NR>(buf, tw, u, a, b);
+            const int g = u / NR, ca = g, cb = g == 0 ? H : BY - g;
+            double2 *row = buf + (u % NR) * P;
+            if (!kPacked && g == 0) { row[M] = make_double2(a[0].y, 0.0); a[0].y = 0.0; }
+#pragma unroll
+            for (int n = 0; n < AY; ++n) { row[ca + BY * n] = a[n]; row[cb + BY * n] = b[n]; }
+        }
+    }
+    __syncthreads();
+}
+
 // c2r of the CTA's columns (natural kz, column-phase layout; CTA 0 with
 // ky = M in slot MC).  Call after a __syncthreads.  On return the CTA holds
 // rows [rank*NR, (rank+1)*NR) of the real plane image: real value (z, y) of
@@ -170,7 +293,7 @@ template <int S> __device__ __forceinline__ double2 tw_get(const double2 *tw, in
 template <class L>
 __device__ __forceinline__ void cl_c2r(double2 *buf, const double2 *tw, int rank) {
     using PN = Plan<L::N>;
-    constexpr int T = L::T, AZ = PN::AZ, BZ = PN::BZ, AY = PN::AY, BY = PN::BY;
+    constexpr int T = L::T, AZ = PN::AZ, BZ = PN::BZ;
     constexpr int MC = L::MC, PZ = L::PZ, NR = L::NR, P = L::P;
     const int tid = threadIdx.x;
     cl_pack_col0<L>(buf, rank);
@@ -232,54 +355,7 @@ __device__ __forceinline__ void cl_c2r(double2 *buf, const double2 *tw, int rank
         }
         cl_sync<L>();   // every row of the plane is in place
     }
-    // real reconstruction and y over AY (slot BY*n1 + n2), twiddle w_M^{n2 k1}
-    constexpr int H = BY / 2;
-#pragma unroll
-    for (int u0 = 0; u0 < NR * H; u0 += T) {
-        const int u = u0 + tid;
-        if (NR * H % T == 0 || u < NR * H) {
-            const int g = u / NR, ca = g, cb = g == 0 ? H : BY - g;
-            double2 *row = buf + (u % NR) * P;
-            double2 a[AY], b[AY];
-#pragma unroll
-            for (int n = 0; n < AY; ++n) { a[n] = row[ca + BY * n]; b[n] = row[cb + BY * n]; }
-            if (g == 0) {   // classes 0 (with ky = 0, M and M/2) and BY/2 mirror onto themselves
-                a[0] = make_double2(a[0].x + a[0].y, a[0].x - a[0].y);
-#pragma unroll
-                for (int n = 1; n < AY / 2; ++n) c2r_pre_pair(a[n], a[AY - n], tw_get<1>(tw, BY * n));
-                a[AY / 2] = make_double2(2.0 * a[AY / 2].x, -2.0 * a[AY / 2].y);
-#pragma unroll
-                for (int n = 0; n < AY / 2; ++n) c2r_pre_pair(b[n], b[AY - 1 - n], tw_get<1>(tw, H + BY * n));
-            } else {
-#pragma unroll
-                for (int n = 0; n < AY; ++n) c2r_pre_pair(a[n], b[AY - 1 - n], tw_get<1>(tw, g + BY * n));
-            }
-            Dft<AY, 1>::run(a);
-            row[ca] = a[0];
-#pragma unroll
-            for (int k1 = 1; k1 < AY; ++k1) row[ca + BY * k1] = cmul(a[k1], tw_get<1>(tw, 2 * ca * k1));
-            Dft<AY, 1>::run(b);
-            row[cb] = b[0];
-#pragma unroll
-            for (int k1 = 1; k1 < AY; ++k1) row[cb + BY * k1] = cmul(b[k1], tw_get<1>(tw, 2 * cb * k1));
-        }
-    }
-    __syncthreads();
-    // y over BY: slot BY*k1 + k2 holds the pair m = k1 + AY*k2
-#pragma unroll
-    for (int u0 = 0; u0 < NR * AY; u0 += T) {
-        const int u = u0 + tid;
-        if (NR * AY % T == 0 || u < NR * AY) {
-            double2 *base = buf + (u % NR) * P + BY * (u / NR);
-            double2 v[BY];
-#pragma unroll
-            for (int n2 = 0; n2 < BY; ++n2) v[n2] = base[n2];
-            Dft<BY, 1>::run(v);
-#pragma unroll
-            for (int k2 = 0; k2 < BY; ++k2) base[k2] = v[k2];
-        }
-    }
-    __syncthreads();
+    rows_c2r<L::N, NR, T, true>(buf, tw);
 }
 
 // The passes of cl_r2c before the last one (z over AZ).
@@ -287,65 +363,17 @@ template <class L>
 __device__ __forceinline__ void cl_r2c_head(double2 *buf, const double2 *tw, int rank) {
     using PN = Plan<L::N>;
     constexpr int T = L::T, AZ = PN::AZ, BZ = PN::BZ, AY = PN::AY, BY = PN::BY;
-    constexpr int MC = L::MC, PZ = L::PZ, NR = L::NR, P = L::P;
+    constexpr int MC = L::MC, PZ = L::PZ, NR = L::NR;
     const int tid = threadIdx.x;
-    // y over BY (slot BY*n1 + n2 holds the pair n1 + AY*n2), twiddle w_M^{n1 k2}
-#pragma unroll
-    for (int u0 = 0; u0 < NR * AY; u0 += T) {
-        const int u = u0 + tid;
-        if (NR * AY % T == 0 || u < NR * AY) {
-            const int n1 = u / NR;
-            double2 *base = buf + (u % NR) * P + BY * n1;
-            double2 v[BY];
-#pragma unroll
-            for (int n2 = 0; n2 < BY; ++n2) v[n2] = base[n2];
-            Dft<BY, -1>::run(v);
-            base[0] = v[0];
-#pragma unroll
-            for (int k2 = 1; k2 < BY; ++k2) base[k2] = cmul(v[k2], tw_get<-1>(tw, 2 * n1 * k2));
-        }
-    }
-    __syncthreads();
-    // y over AY (column BY*k1 + k2) and the real split
-    constexpr int H = BY / 2, TOT = NR * H, K2 = (TOT + T - 1) / T;
-    auto y2 = [&](int u, double2 (&a)[AY], double2 (&b)[AY]) {
-        const int g = u / NR, ca = g, cb = g == 0 ? H : BY - g;
-        const double2 *row = buf + (u % NR) * P;
-#pragma unroll
-        for (int n = 0; n < AY; ++n) { a[n] = row[ca + BY * n]; b[n] = row[cb + BY * n]; }
-        Dft<AY, -1>::run(a);
-        Dft<AY, -1>::run(b);
-        if (g == 0) {   // ky = 0 and M, both real, stay packed as ky = 0 + i ky = M
-            a[0] = make_double2(a[0].x + a[0].y, a[0].x - a[0].y);
-#pragma unroll
-            for (int n = 1; n < AY / 2; ++n) r2c_post_pair(a[n], a[AY - n], tw_get<-1>(tw, BY * n));
-            a[AY / 2].y = -a[AY / 2].y;
-#pragma unroll
-            for (int n = 0; n < AY / 2; ++n) r2c_post_pair(b[n], b[AY - 1 - n], tw_get<-1>(tw, H + BY * n));
-        } else {
-#pragma unroll
-            for (int n = 0; n < AY; ++n) r2c_post_pair(a[n], b[AY - 1 - n], tw_get<-1>(tw, g + BY * n));
-        }
-    };
+    rows_r2c_1<L::N, NR, T>(buf, tw);
     if constexpr (L::C == 1) {
-#pragma unroll
-        for (int u0 = 0; u0 < TOT; u0 += T) {
-            const int u = u0 + tid;
-            if (TOT % T == 0 || u < TOT) {
-                double2 a[AY], b[AY];
-                y2(u, a, b);
-                const int g = u / NR, ca = g, cb = g == 0 ? H : BY - g;
-                double2 *row = buf + (u % NR) * P;
-#pragma unroll
-                for (int n = 0; n < AY; ++n) { row[ca + BY * n] = a[n]; row[cb + BY * n] = b[n]; }
-            }
-        }
-        __syncthreads();
+        rows_r2c_2<L::N, NR, T, true>(buf, tw);
     } else {
+        constexpr int H = BY / 2, TOT = NR * H, K2 = (TOT + T - 1) / T;
         double2 a[K2][AY], b[K2][AY];
 #pragma unroll
         for (int k = 0; k < K2; ++k)
-            if (TOT % T == 0 || tid + k * T < TOT) y2(tid + k * T, a[k], b[k]);
+            if (TOT % T == 0 || tid + k * T < TOT) row_unit_r2c<L::N, NR>(buf, tw, tid + k * T, a[k], b[k]);
         cl_sync<L>();   // every CTA of the plane has read its rows: buffers may be rewritten
 #pragma unroll
         for (int k = 0; k < K2; ++k) {

@@ -706,7 +706,6 @@ int scalar_kernels_per_step(const Geo &g) {
 
 template <int N>
 static cudaError_t set_scalar_attrs() {
-    const int maxs = (int)PL<N>::SMEM;
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(k_sa<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SL<N>::SMEM)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_snl<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NL<N>::SMEM)) != cudaSuccess) return e;
