@@ -617,13 +617,14 @@ def run_gpu(args):
     # FP64 arithmetic: the reference's transform count (31 plane FFTs per
     # x-plane, 2.5 n log2 n flops each for a real n-point plane) and the
     # count this engine executes (25 plane transforms per x-plane; five
-    # circulant line solves per (ky,kz) line, each a forward and an inverse
-    # complex x-FFT of 5 nx log2 nx flops), against the measured DFMA peak
+    # circulant line solves per (ky,kz) line, each two complex recurrences of
+    # two multiply-adds per plane and direction and about 10 per lane to join
+    # the lanes' blocks), against the measured DFMA peak
     import math
     nplane = s.my * mz
     f_plane = 2.5 * nplane * math.log2(nplane)
     f_ref = 31 * nx * f_plane
-    f_exec = 25 * nx * f_plane + (my2 * mz) * 5 * 2 * 5 * nx * math.log2(nx)
+    f_exec = 25 * nx * f_plane + (my2 * mz) * 5 * (16 * nx + 40 * 32)
     fp_peak, fp_ms = C.c_double(), C.c_double()
     fp64 = None
     if lib.pibm_fp64_peak(C.byref(fp_peak), C.byref(fp_ms)) == 0:

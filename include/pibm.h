@@ -30,7 +30,7 @@ extern "C" {
 #define PIBM_OK                   0
 #define PIBM_ERR_ARG            (-1)  /* bad argument / unsupported option                         */
 #define PIBM_ERR_BLOWUP         (-2)  /* norm_drag > 1e6: boundary_condition.F90:874-884            */
-#define PIBM_ERR_PIVOT          (-3)  /* zero pivot in Thomas: tridiagonal.F90:62,72-76             */
+#define PIBM_ERR_PIVOT          (-3)  /* zero pivot: tridiagonal.F90:62,72-76; no system reaches it  */
 #define PIBM_ERR_NAN            (-4)  /* non-finite state detected                                  */
 #define PIBM_ERR_DEM_MOVE       (-5)  /* particle moved >= radius in one DEM sub-step: collision_mod.F90:1421-1428 */
 #define PIBM_ERR_NEIGH_OVERFLOW (-6)  /* neighbour list overflow: collision_mod.F90:845-848          */

@@ -15,8 +15,8 @@
 // terms (in the u tiles) with every rounding written out (psrc_term_rt,
 // cadd_rn), so the results are bitwise those of b_lines.  u and p leave
 // through tensor-map stores of the tile's work tiles.  Tiles are handed out
-// dynamically (an atomic ticket), so the block that draws the (0,0) line,
-// whose Thomas solves are serial, takes fewer tiles.
+// dynamically (an atomic ticket), so a block that starts late or draws lines
+// with more doubling steps takes fewer tiles.
 //
 // Every slab and work tile is a [i][line] box with the 64-byte swizzle: line
 // l of plane i sits at byte i*64 + 16*(l ^ ((i >> 1) & 3)), so a warp reading
