@@ -89,7 +89,7 @@ struct pibm_handle {
     cudaGraphExec_t sgraph[3][2] = {};                    // RK3: one stage per rks and nl parity (pibm_step)
     int step_calls = 0;
     Scal *hsc = nullptr;        // pinned copy of the device scalars (a pageable one is staged by the driver)
-    double *hpart = nullptr;    // pinned staging of get_particles: pres, visc, ptot, force, xc, vel
+    double *hpart = nullptr;    // staging of get_particles behind it: pres, visc, ptot, force, xc, vel
     unsigned geo_ver = 0; // bumped whenever the Geo copies change (graphs hold them by value)
     int cur = 0;          // buffer index the next step writes its nonlinear term to
     int device = 0;
@@ -120,7 +120,6 @@ struct pibm_handle {
         for (auto &gx : graph) if (gx) cudaGraphExecDestroy(gx);
         for (auto &st : sgraph) for (auto &gx : st) if (gx) cudaGraphExecDestroy(gx);
         if (hsc) { cudaHostUnregister(hsc); free(hsc); }
-        if (hpart) cudaFreeHost(hpart);
         if (stream) cudaStreamDestroy(stream);
         if (ss.side) cudaStreamDestroy(ss.side);
         if (ss.scal) cudaStreamDestroy(ss.scal);
@@ -232,16 +231,21 @@ extern "C" {
 
 const char *pibm_last_error(void) { return g_last_error.c_str(); }
 
-// A page of its own, registered: cudaMallocHost maps a whole new chunk when no
-// other pinned memory is held (1 to 2 ms per handle created, and 0.4 to free).
-static cudaError_t pin_scalars(Scal **p) {
+// The handle's pinned read-back memory, pages of its own registered with it: a
+// page for the scalars, then the particle staging.  cudaMallocHost maps a whole
+// new chunk when no other pinned memory is held: 1 to 2 ms per handle created
+// and 0.4 to free for the scalars, 1.1 to 3.7 ms in the first read-back of the
+// particles (registered: 0.05).
+static cudaError_t pin_readback(int nbody, Scal **sc, double **part) {
     constexpr size_t page = 4096;
     static_assert(sizeof(Scal) <= page, "one page");
-    void *q = aligned_alloc(page, page);
+    const size_t bytes = page + (18 * (size_t)nbody * sizeof(double) + page - 1) / page * page;
+    void *q = aligned_alloc(page, bytes);
     if (!q) return cudaErrorMemoryAllocation;
-    const cudaError_t e = cudaHostRegister(q, page, cudaHostRegisterDefault);
+    const cudaError_t e = cudaHostRegister(q, bytes, cudaHostRegisterDefault);
     if (e != cudaSuccess) { free(q); return e; }
-    *p = (Scal *)q;
+    *sc = (Scal *)q;
+    *part = (double *)((char *)q + page);
     return cudaSuccess;
 }
 
@@ -259,7 +263,7 @@ int pibm_create(const pibm_params *prm, const pibm_particles *parts, pibm_handle
         if (e != cudaSuccess) { rc = fail(PIBM_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)); return false; }
         return true;
     };
-    if (!guard(cudaGetDevice(&h->device), "cudaGetDevice") || !guard(pin_scalars(&h->hsc), "pinned scalars") || !guard(configure_kernels(S.my), "configure_kernels") ||
+    if (!guard(cudaGetDevice(&h->device), "cudaGetDevice") || !guard(pin_readback(S.nbody, &h->hsc, &h->hpart), "pinned read-back") || !guard(configure_kernels(S.my), "configure_kernels") ||
         !guard(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
         !guard(cudaStreamCreateWithFlags(&h->ss.side, cudaStreamNonBlocking), "cudaStreamCreate") ||
         !guard(cudaStreamCreateWithFlags(&h->ss.scal, cudaStreamNonBlocking), "cudaStreamCreate") ||
@@ -660,7 +664,6 @@ int pibm_get_particles(pibm_handle *h, double *pres, double *visc, double *force
     if (!h) return fail(PIBM_ERR_ARG, "null handle");
     const size_t n = (size_t)h->S.nbody * 3;
     if (n == 0) return PIBM_OK;
-    if (!h->hpart) CUDA_OR_FAIL(cudaMallocHost(&h->hpart, 6 * n * sizeof(double)));
     double *st = h->hpart;
     if (pres || visc || force) CUDA_OR_FAIL(cudaMemcpyAsync(st, h->b.pres, 4 * n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     if (h->g.moving) {   // the positions and velocities the DEM has advanced

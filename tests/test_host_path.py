@@ -1,0 +1,61 @@
+"""The host's path through the entry points, without a GPU: the engine runs in
+a child process on a preloaded CUDA runtime (fake_cudart.c) whose kernels do
+nothing and whose calls are counted, so what a call allocates, captures and
+launches is known exactly."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+from pureibm_ps2d_fd1d_b200 import build
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+PRELUDE = """
+import ctypes as C
+import numpy as np
+import pureibm_ps2d_fd1d_b200 as pk
+from pureibm_ps2d_fd1d_b200 import config
+fake = C.CDLL(FAKE)
+fake.fake_count.argtypes, fake.fake_count.restype = [C.c_char_p], C.c_long
+fake.fake_fail_launch.argtypes, fake.fake_fail_launch.restype = [C.c_long], None
+count = lambda what: fake.fake_count(what.encode())
+lib = pk.load_library()
+def solver(**kw):
+    prm, xc = config.random_array(my=32, dia_cells=8, nbody=3, seed=1, mc_moves=20)
+    prm.update(kw)
+    return pk.Solver(config.make_params(prm), xc)
+"""
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    build.build()
+    so = str(tmp_path_factory.mktemp("fake") / "libfakecudart.so")
+    subprocess.run(["gcc", "-O1", "-std=c99", "-w", "-shared", "-fPIC", "-o", so, os.path.join(HERE, "fake_cudart.c")], check=True)
+
+    def run(body):
+        env = dict(os.environ, LD_PRELOAD=so, PYTHONPATH=os.path.dirname(HERE))
+        src = "FAKE = %r\n" % so + PRELUDE + textwrap.dedent(body)
+        p = subprocess.run([sys.executable, "-c", src], env=env, capture_output=True, text=True, timeout=300)
+        assert p.returncode == 0, p.stdout + p.stderr
+    return run
+
+
+def test_first_read_back_of_the_particles_pins_nothing(host):
+    """get_particles() stages through memory pinned with the handle: mapping a
+    chunk of pinned memory costs 1 to 4 ms, fifty times the read-back."""
+    host("""
+    s = solver()
+    s.step()
+    before = count("HostAlloc"), count("HostRegister")
+    pres, visc, force, xc, vel = s.get_particles()
+    assert (count("HostAlloc"), count("HostRegister")) == before
+    assert xc.shape == (3, 3) and not pres.any()
+    for my in (1, 2):   # created and closed again
+        t = solver()
+        t.get_particles()
+        t.close()
+    assert count("HostAlloc") == 0
+    """)
