@@ -87,7 +87,7 @@ struct pibm_handle {
     cudaStream_t stream = nullptr;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};        // a time step per nl parity (pibm_run)
     cudaGraphExec_t sgraph[3][2] = {};                    // RK3: one stage per rks and nl parity (pibm_step)
-    int step_calls = 0;
+    int direct_steps = 0;       // time steps pibm_step has launched directly since the graphs were dropped
     Scal *hsc = nullptr;        // pinned copy of the device scalars (a pageable one is staged by the driver)
     double *hpart = nullptr;    // staging of get_particles behind it: pres, visc, ptot, force, xc, vel
     unsigned geo_ver = 0; // bumped whenever the Geo copies change (graphs hold them by value)
@@ -134,6 +134,7 @@ struct pibm_handle {
 static void drop_graphs(pibm_handle *h) {
     for (auto &gx : h->graph) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
     for (auto &st : h->sgraph) for (auto &gx : st) if (gx) { cudaGraphExecDestroy(gx); gx = nullptr; }
+    h->direct_steps = 0;
     ++h->geo_ver;
 }
 
@@ -458,17 +459,24 @@ static int fill_report(pibm_handle *h, pibm_step_report *rep) {
     return PIBM_OK;
 }
 
+// Time steps pibm_step launches directly before it captures the stages it then
+// replays.  A replayed stage saves the host 20 us (32 / 64 / 128^3: 100 / 136 /
+// 555 us launched, 80 / 118 / 537 replayed) and a time step's two parities cost
+// 230 us each to capture and instantiate: they are earned back in 23 steps, so
+// a loop that ends, or drops its graphs (pibm_set_desired_means,
+// pibm_set_tuning), before that never pays for them, and one that goes on has
+// lost no more than a capture costs.
+constexpr int kDirectSteps = 24;
+
 int pibm_step(pibm_handle *h, int rks, pibm_step_report *rep) {
     if (!h) return fail(PIBM_ERR_ARG, "null handle");
     if (rks < 1 || rks > h->itrmax) return fail(PIBM_ERR_ARG, h->itrmax == 1 ? "AB2 has a single stage (rks = 1)" : "rks must be 1, 2 or 3 (RK3)");
     if (rks != h->next_rks) return fail(PIBM_ERR_ARG, "stages must run in the order rks = 1..itrmax");
     // a host that steps in a loop replays a graph of the stage: its dozen
     // launches and event waits cost the CPU more than a small grid's step takes
-    // the GPU (the driver loop at 32^3: 181 us per iteration, 118 with the pinned
-    // read-backs); the first calls launch directly, so a few steps do not pay
-    // for a capture
-    if (++h->step_calls > 2) {
-        cudaGraphExec_t &gx = h->itrmax == 1 ? h->graph[h->cur] : h->sgraph[rks - 1][h->cur];
+    // the GPU
+    cudaGraphExec_t &gx = h->itrmax == 1 ? h->graph[h->cur] : h->sgraph[rks - 1][h->cur];
+    if (gx || h->direct_steps >= kDirectSteps) {
         if (!gx) {
             cudaGraph_t gr;
             CUDA_OR_FAIL(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
@@ -481,6 +489,7 @@ int pibm_step(pibm_handle *h, int rks, pibm_step_report *rep) {
         CUDA_OR_FAIL(cudaGraphLaunch(gx, h->stream));
     } else {
         enqueue_step(h->gs[rks - 1], h->b, h->cur, h->stream, nullptr, &h->ss);
+        if (rks == h->itrmax) ++h->direct_steps;
     }
     CUDA_OR_FAIL(cudaGetLastError());
     h->cur ^= 1;

@@ -59,3 +59,43 @@ def test_first_read_back_of_the_particles_pins_nothing(host):
         t.close()
     assert count("HostAlloc") == 0
     """)
+
+
+def test_step_captures_only_what_a_long_loop_replays(host):
+    """A capture costs what a dozen replays save: short loops, and loops that
+    change the run between steps (which drops the graphs), launch directly; long
+    ones replay each stage and parity from one capture, RK3 by time steps and not by stages."""
+    host("""
+    means = np.array([1e-3, 0.0, 0.0])
+    dp = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))
+    for rk3 in (False, True):
+        stages = 3 if rk3 else 1
+        def steps(s, n):
+            for _ in range(n):
+                for rks in range(1, stages + 1):
+                    s.step(rks)
+        base = count("Instantiate")
+        s = solver(rk3=rk3)
+        steps(s, 20)
+        assert count("Instantiate") == base
+        for _ in range(60):   # each drops the graphs
+            assert lib.pibm_set_desired_means(s.h, dp(means), dp(means)) == 0
+            steps(s, 1)
+        assert count("Instantiate") == base
+        steps(s, 60)
+        made, launched = count("Instantiate"), count("Launch")
+        assert made == base + 2 * stages
+        steps(s, 60)          # replayed: no direct launch, no further capture
+        assert (count("Instantiate"), count("Launch")) == (made, launched)
+        assert lib.pibm_set_tuning(s.h, s.tuning()["lines_per_cta"]) == 0
+        steps(s, 20)
+        assert count("Instantiate") == made and count("Launch") > launched
+        s.close()
+        t = solver(rk3=rk3)   # an AB2 step is the graph that pibm_run has captured
+        t.run(2)
+        assert count("Instantiate") == made + 2
+        launched = count("Launch")
+        steps(t, 3)
+        assert count("Instantiate") == made + 2 and (count("Launch") == launched) == (not rk3)
+        t.close()
+    """)
