@@ -222,6 +222,26 @@ static int setup_moving(pibm_handle *h) {
     return PIBM_OK;
 }
 
+// Captures what enqueue() puts on stream s into an executable graph.  A launch
+// that fails within a capture leaves its error behind and the capture valid
+// without it, so the error is taken here: such a graph is not kept.  (An error
+// that the program left behind earlier is not the capture's.)
+template <class F>
+static int capture(cudaStream_t s, cudaGraphExec_t *gx, F enqueue) {
+    const bool clean = cudaPeekAtLastError() == cudaSuccess;
+    CUDA_OR_FAIL(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    const int rc = enqueue();
+    cudaGraph_t gr = nullptr;
+    cudaError_t e = cudaStreamEndCapture(s, &gr);
+    if (clean) { const cudaError_t el = cudaGetLastError(); if (e == cudaSuccess) e = el; }
+    if (e == cudaSuccess && !rc) e = cudaGraphInstantiate(gx, gr, 0);
+    if (gr) cudaGraphDestroy(gr);
+    if (e != cudaSuccess || rc) *gx = nullptr;
+    if (rc) return rc;
+    CUDA_OR_FAIL(e);
+    return PIBM_OK;
+}
+
 // One time step = stages rks = 1..itrmax; stage k writes the nonlinear term
 // into buffer cur ^ (k & 1) (the onl = nl swap of every nonlinear call).
 static void enqueue_time_step(pibm_handle *h, int cur, cudaStream_t s, const StepStreams *ss) {
@@ -478,13 +498,11 @@ int pibm_step(pibm_handle *h, int rks, pibm_step_report *rep) {
     cudaGraphExec_t &gx = h->itrmax == 1 ? h->graph[h->cur] : h->sgraph[rks - 1][h->cur];
     if (gx || h->direct_steps >= kDirectSteps) {
         if (!gx) {
-            cudaGraph_t gr;
-            CUDA_OR_FAIL(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-            enqueue_step(h->gs[rks - 1], h->b, h->cur, h->stream, nullptr, &h->ss);
-            CUDA_OR_FAIL(cudaStreamEndCapture(h->stream, &gr));
-            const cudaError_t e = cudaGraphInstantiate(&gx, gr, 0);
-            cudaGraphDestroy(gr);
-            CUDA_OR_FAIL(e);
+            const int rc = capture(h->stream, &gx, [&]() -> int {
+                enqueue_step(h->gs[rks - 1], h->b, h->cur, h->stream, nullptr, &h->ss);
+                return PIBM_OK;
+            });
+            if (rc) return rc;
         }
         CUDA_OR_FAIL(cudaGraphLaunch(gx, h->stream));
     } else {
@@ -502,12 +520,11 @@ int pibm_run(pibm_handle *h, int nsteps, pibm_step_report *last) {
     if (h->next_rks != 1) return fail(PIBM_ERR_ARG, "pibm_run starts at a step boundary (finish the rks stages with pibm_step)");
     for (int par = 0; par < 2; ++par) {
         if (h->graph[par]) continue;
-        cudaGraph_t gr;
-        CUDA_OR_FAIL(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_time_step(h, par, h->stream, &h->ss);
-        CUDA_OR_FAIL(cudaStreamEndCapture(h->stream, &gr));
-        CUDA_OR_FAIL(cudaGraphInstantiate(&h->graph[par], gr, 0));
-        cudaGraphDestroy(gr);
+        const int rc = capture(h->stream, &h->graph[par], [&]() -> int {
+            enqueue_time_step(h, par, h->stream, &h->ss);
+            return PIBM_OK;
+        });
+        if (rc) return rc;
     }
     for (int s = 0; s < nsteps; ++s) {
         CUDA_OR_FAIL(cudaGraphLaunch(h->graph[h->cur], h->stream));
@@ -1453,34 +1470,32 @@ static int batch_graphs(pibm_batch *bt) {
     bt->captured_fused = bt->fused;
     batch_members(bt);
     for (int par = 0; par < 2; ++par) {
-        cudaGraph_t gr;
-        CUDA_OR_FAIL(cudaStreamBeginCapture(bt->stream, cudaStreamCaptureModeThreadLocal));
-        // the groups one after another (run side by side, their launches
-        // compete for SMs and L2 and the step takes longer), then the others
-        if (bt->fused)
-            for (auto &G : bt->groups)
-                for (int k = 0; k < G.itrmax; ++k)
-                    enqueue_batch_step(G.n, G.sets[(size_t)par * G.itrmax + k], G.shape, bt->stream, G.side, G.fork,
-                                       G.join);
-        CUDA_OR_FAIL(cudaEventRecord(bt->fork, bt->stream));
-        // members whose plane kernels alone fill the GPU (nx*C CTAs per transform item
-        // of at least one per SM slot) form one chain, one after the other; the
-        // smaller members run as parallel branches beside that chain
-        int prev_big = -1;
-        for (int q = 0; q < n; ++q) {
-            if (bt->fused && bt->in_group[q]) continue;
-            pibm_handle *h = bt->members[q];
-            const bool big = h->g.my >= 128;
-            CUDA_OR_FAIL(cudaStreamWaitEvent(h->stream, (big && prev_big >= 0) ? bt->join[prev_big] : bt->fork, 0));
-            enqueue_time_step(h, bt->base[q] ^ par, h->stream, &h->ss);
-            CUDA_OR_FAIL(cudaEventRecord(bt->join[q], h->stream));
-            CUDA_OR_FAIL(cudaStreamWaitEvent(bt->stream, bt->join[q], 0));
-            if (big) prev_big = q;
-        }
-        CUDA_OR_FAIL(cudaStreamEndCapture(bt->stream, &gr));
-        const cudaError_t e = cudaGraphInstantiate(&bt->graph[par], gr, 0);
-        cudaGraphDestroy(gr);
-        CUDA_OR_FAIL(e);
+        const int rc = capture(bt->stream, &bt->graph[par], [&]() -> int {
+            // the groups one after another (run side by side, their launches
+            // compete for SMs and L2 and the step takes longer), then the others
+            if (bt->fused)
+                for (auto &G : bt->groups)
+                    for (int k = 0; k < G.itrmax; ++k)
+                        enqueue_batch_step(G.n, G.sets[(size_t)par * G.itrmax + k], G.shape, bt->stream, G.side, G.fork,
+                                           G.join);
+            CUDA_OR_FAIL(cudaEventRecord(bt->fork, bt->stream));
+            // members whose plane kernels alone fill the GPU (nx*C CTAs per transform item
+            // of at least one per SM slot) form one chain, one after the other; the
+            // smaller members run as parallel branches beside that chain
+            int prev_big = -1;
+            for (int q = 0; q < n; ++q) {
+                if (bt->fused && bt->in_group[q]) continue;
+                pibm_handle *h = bt->members[q];
+                const bool big = h->g.my >= 128;
+                CUDA_OR_FAIL(cudaStreamWaitEvent(h->stream, (big && prev_big >= 0) ? bt->join[prev_big] : bt->fork, 0));
+                enqueue_time_step(h, bt->base[q] ^ par, h->stream, &h->ss);
+                CUDA_OR_FAIL(cudaEventRecord(bt->join[q], h->stream));
+                CUDA_OR_FAIL(cudaStreamWaitEvent(bt->stream, bt->join[q], 0));
+                if (big) prev_big = q;
+            }
+            return PIBM_OK;
+        });
+        if (rc) return rc;
     }
     return PIBM_OK;
 }

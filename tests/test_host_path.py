@@ -99,3 +99,49 @@ def test_step_captures_only_what_a_long_loop_replays(host):
         assert count("Instantiate") == made + 2 and (count("Launch") == launched) == (not rk3)
         t.close()
     """)
+
+
+def test_launch_that_fails_within_a_capture_is_reported(host):
+    """A launch that fails while a step is captured fails the call, and the graph
+    without it is not kept: the next call captures a whole one."""
+    host("""
+    def fails(call):
+        try:
+            call()
+        except pk.PibmError as e:
+            assert e.code == -8, e
+            return
+        raise AssertionError("the failed launch was not reported")
+    s = solver()
+    fake.fake_fail_launch(3)
+    fails(lambda: s.run(2))
+    assert count("Instantiate") == 0 and count("GraphLaunch") == 0
+    per_step = s.info.kernels_per_step
+    before = count("Capture")
+    s.run(2)
+    assert count("Instantiate") == 2 and count("GraphLaunch") == 2
+    assert count("Capture") - before == 2 * per_step
+    s.close()
+
+    t = solver(rk3=True)
+    for _ in range(24):
+        for rks in (1, 2, 3):
+            t.step(rks)
+    made, replayed = count("Instantiate"), count("GraphLaunch")
+    fake.fake_fail_launch(2)
+    fails(lambda: t.step(1))
+    assert (count("Instantiate"), count("GraphLaunch")) == (made, replayed)
+    t.step(1)
+    assert (count("Instantiate"), count("GraphLaunch")) == (made + 1, replayed + 1)
+    t.close()
+
+    prm, xc = config.random_array(my=32, dia_cells=8, nbody=3, seed=1, mc_moves=20)
+    b = pk.Batch([(dict(prm), xc)] * 2 + [(dict(prm, iscalon=1, pr_or_sc_nu=0.7, phisurf=1.0, phistream=0.0,
+                                                initialize_zero=False), xc)])
+    made = count("Instantiate")
+    fake.fake_fail_launch(5)
+    fails(lambda: b.run(1))
+    assert count("Instantiate") == made
+    b.run(1)
+    assert count("Instantiate") == made + 2
+    """)
