@@ -483,7 +483,7 @@ struct MarchWarp {
 // Shared-memory layout of a CTA (the same in every CTA of the cluster).
 struct MarchMem {
     double *P[2], *V[2], *pcand, *hyd;   // [3*l + d] of all particles; of the CTA's own: candidates' base, fluid force / mass
-    int *cell[2], *flags, *pcs;          // packed cells of all; 3 rotating flag words; contact counts held in either global buffer
+    int *cell[2], *flags, *pcs;          // packed cells of all; 3 rotating flag words and the sub-step count; contact counts held in either global buffer
     unsigned short *nb, *cand;
     unsigned char *nbc, *cdc;
     MarchWarp *w;
@@ -560,8 +560,6 @@ __global__ void __launch_bounds__(1024, 1) k_dem_march(Mov m, Scal *sc, const do
     const int N = m.N, MX = m.maxn, slots = (N + ctas - 1) / ctas;   // particle L: CTA L % ctas, slot L / ctas
     MarchMem S(march_s, N, slots, MX, nw);
     MarchWarp &W = S.w[wid];
-    const bool failed = sc->status != 0;   // set by earlier kernels only: the same for every thread
-    const int F = failed ? 0 : m.factor[0];
     const double dts = m.dts[0];
     const int d3 = lane % 3;               // this lane's direction in CFNEWVALUES
     const double fa = sc->frame_accln[d3], gm = (sc->mpg[d3] * m.pvol) / m.pmass;
@@ -581,12 +579,18 @@ __global__ void __launch_bounds__(1024, 1) k_dem_march(Mov m, Scal *sc, const do
         if (lane == 0) { S.nbc[k] = (unsigned char)nc; S.pcs[k] = m.pncnt[L]; S.pcs[slots + k] = -1; }
     }
     if (threadIdx.x < 3) S.flags[threadIdx.x] = 0;
+    // The sub-steps to take, none after a failure: every thread must come to the
+    // cluster's barriers equally often, so one thread reads the status for all
+    // (a kernel beside this one may set it at any time).
+    if (rank == 0 && threadIdx.x == 3) S.flags[3] = sc->status != 0 ? 0 : m.factor[0];
     cl.sync();
+    if (rank != 0 && threadIdx.x == 0) S.flags[3] = cl.map_shared_rank(S.flags, 0)[3];
+    __syncthreads();
     auto raise = [&](int f, int word) {   // in every CTA's copy of the flag word
         for (int r = 0; r < ctas; ++r) atomicOr(cl.map_shared_rank(S.flags, r) + word, f);
     };
     int s = 0, c = 0;
-    for (; s < F; ++s, c ^= 1) {
+    for (; s < *(volatile int *)(S.flags + 3); ++s, c ^= 1) {
         double *const Pc = S.P[c], *const Vc = S.V[c], *const Pn = S.P[c ^ 1], *const Vn = S.V[c ^ 1];
         int *const Cn = S.cell[c ^ 1];
         int *const gl = c ? m.pn2 : m.pn, *const gv = c ? m.pv2 : m.pv, *const gc = c ? m.pncnt2 : m.pncnt;
