@@ -30,6 +30,7 @@ void enqueue_batch_step(int n, const MemberSet &ms, const BatchShape &bs, cudaSt
                         cudaEvent_t fork, cudaEvent_t join);
 void enqueue_dem_init(const Mov &m, Scal *sc, cudaStream_t s);
 cudaError_t configure_moving_kernels(const Mov &m);
+bool dem_march(const Mov &m);
 void enqueue_c2r(const Geo &g, const double2 *a, double *b, int nplanes, cudaStream_t s);
 void enqueue_r2c(const Geo &g, const double *a, double2 *b, int nplanes, cudaStream_t s);
 void enqueue_f2d(const double2 *f, double2 *d, int nx, int nxf, int PS, int ncomp, cudaStream_t s);
@@ -157,6 +158,7 @@ static int setup_moving(pibm_handle *h) {
     m.kn = S.dem_kn; m.eta_n = S.dem_eta_n; m.rad = S.dem_rad; m.pmass = S.dem_pmass; m.pvol = S.dem_pvol;
     m.rhof = h->prm.rhof; m.dtsolid = S.dem_dtsolid; m.max_radius = S.dem_rad;
     m.max_factor = m.soft ? std::max(1, (int)(S.dt / m.dtsolid)) : 1;
+    m.march = dem_march(m);
     m.kmax = S.my >= 256 ? 32 : 48;
     if (m.ncell > 8192 || 3 * m.ncell + 1 + N > 40000)
         return fail(PIBM_ERR_ARG, "moving particles: coarse DEM grid or particle count too large for the binning kernel");

@@ -80,6 +80,7 @@ struct Scal {
 // reference's (collision_mod.F90 NEIGHBOURS / PN / PV).
 struct Mov {
     int N, maxn, soft, max_factor;
+    int march;                                 // all sub-steps of a flow step in one launch (dem_march)
     int cx, cy, cz, ncell;            // coarse grid nodes per direction; physical cells 2..c
     double dxc, dyc, dzc, LXs, LYs, LZs, XL, YL, ZL;
     double kn, eta_n, rad, pmass, pvol, rhof, dtsolid, max_radius;

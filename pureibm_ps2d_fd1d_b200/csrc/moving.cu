@@ -11,7 +11,8 @@
 // The reference keeps the contact lists with one sequential loop over the
 // particles.  Here all sub-steps of a flow step run in one launch of one
 // thread-block cluster (k_dem_march), up to kMarchMax particles; larger
-// systems, which need the whole GPU, take three launches per sub-step:
+// systems, which need the whole GPU, and larger ones with few sub-steps take
+// three launches per sub-step:
 //   k_dem_update  one thread per particle L: every pair (J, L) is evaluated by
 //                 both its threads with the same arithmetic; L applies what the
 //                 serial loop does to L's list at J's turn (J < L), then at
@@ -468,9 +469,16 @@ __global__ void __launch_bounds__(32 * kSearchWarps) k_dem_search(Mov m, Scal *s
 // barrier per sub-step with 43 particles on eight SMs, 4.9 us against 16.5 us
 // for the three launches.
 // ============================================================================
-// Particles.  Eight SMs take 41 us per sub-step with 1202 (their FP64 pipes are
-// full), the three launches over the whole GPU 33; the lines cross near 700.
-constexpr int kMarchMax = 512;
+// Where one launch per flow step is the shorter one (dem_march).  Eight SMs take
+// 41 us per sub-step with 1202 particles (their FP64 pipes are full), the three
+// launches over the whole GPU 33; with 512 it is 23 against 33, and fewer gain
+// more.  But the march forms all candidates once per flow step, which takes
+// eight SMs longer than it takes the GPU, and from 256 particles on needs more
+// sub-steps to share it.  Steps of a suspension at 64^3, d = 6, by launches / by
+// the march: 512 particles 1.16 at 26 sub-steps, 1.07 at 11, 1.02 at 6, 0.97 at 4 and 1;
+// 448: 1.05 at 7, 0.98 at 5; 384: 1.02 at 5, 0.98 at 3; 320: 1.02 at 4, 1.00 at 3, 0.96 at 1;
+// 256: 1.14 at 5, 1.00 at 1; 128^3, d = 12, 400 particles: 1.04 at 13, 0.99 at 6.
+constexpr int kMarchMax = 512, kMarchAny = 256, kMarchPerSubStep = 32;
 constexpr int kMarchCtas = 8;      // portable cluster size
 constexpr int kMaxCand = 48;
 constexpr double kSkin = 0.4;      // in particle radii, on top of 2.4 (the search radius)
@@ -1198,7 +1206,6 @@ MarchShape march_shape(const Mov &m) {
     t.smem = MarchMem::bytes(m.N, slots, m.maxn, t.warps);
     return t;
 }
-bool use_march(const Mov &m) { return m.soft && m.N <= kMarchMax && m.maxn < kMaxList && m.cx < 1024 && m.cy < 1024 && m.cz < 1024; }
 void launch_march(const Mov &m, Scal *sc, const double *pres, const double *visc, cudaStream_t s) {
     const MarchShape t = march_shape(m);
     cudaLaunchConfig_t cfg = {};
@@ -1222,7 +1229,7 @@ void enqueue_moving_t(const Geo &g, const Mov &m, Scal *sc, const double *pres, 
     k_dem_start<<<1, 32, 0, s>>>(m, sc);
     if (m.soft) {
         const size_t bin_smem = (size_t)(3 * m.ncell + 1 + m.N) * sizeof(int);
-        if (use_march(m)) launch_march(m, sc, pres, visc, s);
+        if (m.march) launch_march(m, sc, pres, visc, s);
         else for (int ifac = 1; ifac <= m.max_factor; ++ifac) {
             k_dem_update<<<(m.N + kUpdWarps - 1) / kUpdWarps, 32 * kUpdWarps, 0, s>>>(m, sc, pres, visc, ifac);
             k_dem_bin<<<1, 1024, bin_smem, s>>>(m, sc, ifac);
@@ -1254,7 +1261,7 @@ void enqueue_moving(const Geo &g, const Mov &m, Scal *sc, const double *pres, co
         case 256: enqueue_moving_t<256>(g, m, sc, pres, visc, s); break;
     }
 }
-int moving_kernels_per_step(const Mov &m) { return 1 + (m.soft && !use_march(m) ? 3 * m.max_factor : 1) + 6; }
+int moving_kernels_per_step(const Mov &m) { return 1 + (m.soft && !m.march ? 3 * m.max_factor : 1) + 6; }
 
 // Scalar geometry of the step (before calc_inner_rev_data) and its spreading.
 void enqueue_moving_scalar(const Geo &g, const Mov &m, Scal *sc, cudaStream_t s) {
@@ -1284,6 +1291,12 @@ void enqueue_dem_init(const Mov &m, Scal *sc, cudaStream_t s) {
     const size_t bin_smem = (size_t)(3 * m.ncell + 1 + m.N) * sizeof(int);
     k_dem_bin<<<1, 1024, bin_smem, s>>>(m, sc, 1);
     k_dem_search<<<(m.N + kSearchWarps - 1) / kSearchWarps, 32 * kSearchWarps, 0, s>>>(m, sc, 1);
+}
+
+// Whether a run's sub-steps go in one launch per flow step (kMarchMax).
+bool dem_march(const Mov &m) {
+    return m.soft && m.N <= kMarchMax && m.N <= kMarchAny + kMarchPerSubStep * (m.max_factor - 1) && m.maxn < kMaxList &&
+           m.cx < 1024 && m.cy < 1024 && m.cz < 1024;
 }
 
 cudaError_t configure_moving_kernels(const Mov &m) {

@@ -145,3 +145,26 @@ def test_launch_that_fails_within_a_capture_is_reported(host):
     b.run(1)
     assert count("Instantiate") == made + 2
     """)
+
+
+def test_dem_in_one_launch_where_its_sub_steps_pay_for_it(host):
+    """Launches per step of soft-sphere runs: one for all sub-steps up to 256
+    spheres, and 32 more for each sub-step after the first up to 512; else
+    three per sub-step."""
+    host("""
+    def launches(n, rhos):
+        prm, _ = config.single_sphere(my=64, dia_cells=6.0, re=20.0)
+        prm.update(imove=1, collision_type="softsphere", rhos=rhos, rhof=1.0, coeff_rest=0.9, initialize_zero=True)
+        s = pk.Solver(config.make_params(prm), config.fcc_subset(n, 64.0, 6.0, np.random.default_rng(n)))
+        before = count("Launch")
+        s.step()
+        made = count("Launch") - before
+        assert made == s.info.kernels_per_step
+        s.close()
+        return made
+    one = launches(1, 1e2)
+    assert [launches(n, 1e2) for n in (256, 257, 512)] == [one] * 3     # 82 sub-steps
+    assert launches(513, 1e2) > one + 3 * 50
+    assert launches(256, 1e9) == one                                    # one sub-step
+    assert [launches(n, 1e9) for n in (257, 512, 513)] == [one + 2] * 3
+    """)
