@@ -592,13 +592,12 @@ __global__ void __launch_bounds__(1024, 1) k_dem_march(Mov m, Scal *sc, const do
     // (a kernel beside this one may set it at any time).
     if (rank == 0 && threadIdx.x == 3) S.flags[3] = sc->status != 0 ? 0 : m.factor[0];
     cl.sync();
-    if (rank != 0 && threadIdx.x == 0) S.flags[3] = cl.map_shared_rank(S.flags, 0)[3];
-    __syncthreads();
+    const int F = cl.map_shared_rank(S.flags, 0)[3];
     auto raise = [&](int f, int word) {   // in every CTA's copy of the flag word
         for (int r = 0; r < ctas; ++r) atomicOr(cl.map_shared_rank(S.flags, r) + word, f);
     };
     int s = 0, c = 0;
-    for (; s < *(volatile int *)(S.flags + 3); ++s, c ^= 1) {
+    for (; s < F; ++s, c ^= 1) {
         double *const Pc = S.P[c], *const Vc = S.V[c], *const Pn = S.P[c ^ 1], *const Vn = S.V[c ^ 1];
         int *const Cn = S.cell[c ^ 1];
         int *const gl = c ? m.pn2 : m.pn, *const gv = c ? m.pv2 : m.pv, *const gc = c ? m.pncnt2 : m.pncnt;
