@@ -1301,14 +1301,14 @@ __global__ void __launch_bounds__(RL<N>::T, RL<N>::MINB) k_ff2rc(Geo g, const do
 // The column and row sweeps of the larger grids (sweep.cuh).
 template <int N> constexpr bool use_sweeps() { return N >= kSweepMin; }
 template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 5) k_cz(Geo g, const double2 *__restrict__ u, const double2 *__restrict__ p, double2 *__restrict__ zf) { b_cz<N>(g, u, p, zf); }
-template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) k_ry(Geo g, const double2 *__restrict__ zf, double *__restrict__ ubcp, double *__restrict__ pbcp, double *__restrict__ omega,
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, Sweep<N>::RBLK) k_ry(Geo g, const double2 *__restrict__ zf, double *__restrict__ ubcp, double *__restrict__ pbcp, double *__restrict__ omega,
                                                                        double *__restrict__ pgr, Scal *__restrict__ sc, double *__restrict__ part) { b_ry<N>(g, zf, ubcp, pbcp, omega, pgr, sc, part); }
-template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) k_rp(Geo g, const double *__restrict__ ubcp, const double *__restrict__ Dx, double2 *__restrict__ pz, Scal *__restrict__ sc) { b_rp<N>(g, ubcp, Dx, pz, sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, Sweep<N>::RBLK) k_rp(Geo g, const double *__restrict__ ubcp, const double *__restrict__ Dx, double2 *__restrict__ pz, Scal *__restrict__ sc) { b_rp<N>(g, ubcp, Dx, pz, sc); }
 template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 4) k_cn(Geo g, const double2 *__restrict__ pz, double2 *nl_new) { b_cn<N>(g, pz, nl_new); }
 template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 4) k_cq(Geo g, const double2 *__restrict__ nl, const double2 *__restrict__ u, const double2 *__restrict__ onl,
                                                                        double2 *__restrict__ qz) { b_cq<N>(g, nl, u, onl, qz); }
-template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) k_rq(Geo g, const double2 *__restrict__ qz, double *__restrict__ Q, Scal *__restrict__ sc) { b_rq<N>(g, qz, Q, sc); }
-template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) k_rf(Geo g, const double *__restrict__ fr, double2 *__restrict__ fz, Scal *__restrict__ sc) { b_rf<N>(g, fr, fz, sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, Sweep<N>::RBLK) k_rq(Geo g, const double2 *__restrict__ qz, double *__restrict__ Q, Scal *__restrict__ sc) { b_rq<N>(g, qz, Q, sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, Sweep<N>::RBLK) k_rf(Geo g, const double *__restrict__ fr, double2 *__restrict__ fz, Scal *__restrict__ sc) { b_rf<N>(g, fr, fz, sc); }
 template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 5) k_cf(Geo g, const double2 *__restrict__ fz, double2 *__restrict__ ff) { b_cf<N>(g, fz, ff); }
 // A launch that may start its prologue while the previous kernel of the stream drains.
 template <typename... KArgs, typename... Args>
@@ -1387,15 +1387,15 @@ __global__ void __launch_bounds__(256, 4) kb_flux(const __grid_constant__ Member
     b_flux<N>(m.g, m.b.ubcp, m.b.Dx, m.b.sc);
 }
 template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 5) kb_cz(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_cz<N>(m.g, m.b.u, m.b.p, m.b.wz); }
-template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) kb_ry(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_ry<N>(m.g, m.b.wz, m.b.ubcp, m.b.pbcp, m.b.omega, m.b.pgr, m.b.sc, m.b.part); }
-template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) kb_rp(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_rp<N>(m.g, m.b.ubcp, m.b.Dx, wz_products<N>(m.b.wz), m.b.sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, Sweep<N>::RBLK) kb_ry(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_ry<N>(m.g, m.b.wz, m.b.ubcp, m.b.pbcp, m.b.omega, m.b.pgr, m.b.sc, m.b.part); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, Sweep<N>::RBLK) kb_rp(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_rp<N>(m.g, m.b.ubcp, m.b.Dx, wz_products<N>(m.b.wz), m.b.sc); }
 template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 4) kb_cn(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_cn<N>(m.g, wz_products<N>(m.b.wz), m.b.nl[m.cur]); }
 template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 4) kb_cq(const __grid_constant__ MemberSet ms) {
     const Member &m = ms.m[blockIdx.z];
     b_cq<N>(m.g, m.b.nl[m.cur], m.b.u, m.b.nl[m.cur ^ 1], wz_q<N>(m.b.wz));
 }
-template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) kb_rq(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_rq<N>(m.g, wz_q<N>(m.b.wz), m.b.Q, m.b.sc); }
-template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, 6) kb_rf(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; if (m.g.nbody == 0) return; b_rf<N>(m.g, m.b.fr, m.b.wz, m.b.sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, Sweep<N>::RBLK) kb_rq(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; b_rq<N>(m.g, wz_q<N>(m.b.wz), m.b.Q, m.b.sc); }
+template <int N> __global__ void __launch_bounds__(Sweep<N>::RT, Sweep<N>::RBLK) kb_rf(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; if (m.g.nbody == 0) return; b_rf<N>(m.g, m.b.fr, m.b.wz, m.b.sc); }
 template <int N> __global__ void __launch_bounds__(Sweep<N>::CT, 5) kb_cf(const __grid_constant__ MemberSet ms) { const Member &m = ms.m[blockIdx.z]; if (m.g.nbody == 0) return; b_cf<N>(m.g, m.b.wz, m.b.ff); }
 template <int N>
 __global__ void __launch_bounds__(NL<N>::T, NL<N>::MINB) kb_nl(const __grid_constant__ MemberSet ms) {

@@ -37,8 +37,11 @@ template <int N> struct Sweep {
     static constexpr int RC = N >= 256 ? 16 : 32;     // rows of a block
     static constexpr int RT = 128, RB = N / RC;       // threads, blocks of a plane
     static constexpr int RSM = (RC * my2 + N) * 16;
+    static constexpr int RBLK = 6;                    // row blocks per SM the register budget is sized for
     static constexpr uint32_t RBYTES = RC * my2 * 16; // rows of a block, spectral or real: N (N+2) doubles = my2 N complex
     static_assert(M % QC == 0 && N % QC == 0 && QC * AZ % CT == 0, "column blocks");
+    // 228 KB per SM, of which each block takes 1 KB beside its own (a barrier is its only static memory)
+    static_assert(RBLK * (RSM + 128 + 1024) <= 228 * 1024, "row blocks");
 };
 // A thread's column: its plane, ky index and offset in a field's planes.
 struct ColPos { int i, j; size_t off; };
@@ -134,7 +137,6 @@ __device__ __forceinline__ void b_ry(const Geo &g, const double2 *__restrict__ z
     constexpr int my2 = W::my2, PS = W::PS, RSP = RP<N>::RSP, nx = N;
     extern __shared__ double2 sm[];
     double2 *buf = sm, *tws = sm + W::RC * my2;
-    __shared__ double scr[32 * 3];
     __shared__ uint64_t mb;
     if (threadIdx.x == 0) mbar_init(&mb, 1);
     for (int t = threadIdx.x; t < N; t += W::RT) tws[t] = g.tw[t];
@@ -182,7 +184,10 @@ __device__ __forceinline__ void b_ry(const Geo &g, const double2 *__restrict__ z
     rows_c2r<N, W::RC, W::RT, false>(buf, tws);
     const size_t roff = (size_t)i * RSP + (size_t)rb * W::RC * (N + 2);
     if (t < 3) {
-        // u + umean; fluid, solid and total sums and max |u| of this block's rows
+        // u + umean; fluid, solid and total sums and max |u| of this block's rows.
+        // Scratch of its own left room for five blocks per SM (fields to real space 1031 -> 958 us).
+        double *scr = (double *)tws;   // the transform's last barrier is behind every thread
+        static_assert(N * sizeof(double2) >= 32 * 3 * sizeof(double), "reduction scratch");
         const double um = sc->umean[t];
         double *b = (double *)buf;
         const uint8_t *fl = g.fluid + roff;
