@@ -9,6 +9,7 @@ import pytest
 
 import pureibm_ps2d_fd1d_b200 as pk
 from pureibm_ps2d_fd1d_b200 import config
+import oracle_ctypes as oc
 
 
 def _members():
@@ -101,19 +102,37 @@ def test_mixed_batch_matches_single_runs_bitwise(fused):
     b.close()
 
 
+#: kSpreadFewNodes of csrc/kernels.cu: launches of at most this many forced
+#: nodes spread with several lanes per node
+FEW_NODES = 20000
+
+
+def _forced_nodes(prm, xc):
+    """Nodes that receive force: where the oracle's first step leaves any."""
+    parts = config.Particles(xc)
+    cpu = oc.OracleSolver(config.make_params(prm), parts.struct)
+    cpu.step()
+    return int(np.count_nonzero(np.any(cpu.get_field(5) != 0.0, axis=0)))
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("my,dia,n,width,limiter,frfl", [(32, 8.0, 1, 2, "none", False), (32, 8.0, 3, 12, "minmod", True),
-                                                         (64, 10.0, 1, 10, "none", False), (64, 7.0, 40, 2, "none", False)])
-def test_spreading_by_lanes_equals_one_thread_per_node_bitwise(my, dia, n, width, limiter, frfl):
+@pytest.mark.parametrize("my,dia,n,width,limiter,frfl,lanes", [
+    (64, 7.0, 40, 4, "none", False, (True, False)), (64, 7.0, 40, 4, "minmod", True, (True, False)),
+    (32, 8.0, 1, 2, "none", False, (True, True)), (32, 8.0, 3, 12, "minmod", True, (True, True)),
+    (64, 10.0, 1, 10, "none", False, (True, True)), (64, 7.0, 40, 2, "none", False, (True, True)),
+    (64, 10.0, 60, 2, "none", False, (False, False))])
+def test_spreading_by_lanes_equals_one_thread_per_node_bitwise(my, dia, n, width, limiter, frfl, lanes):
     """Launches of few forced nodes spread with several lanes per node, the
-    others with one thread: a narrow batch and its members alone take the
-    former, a wide batch and an array of 40 spheres the latter, and every
-    combination ends at the same bits."""
+    others with one thread per node.  `lanes`: which form a member takes alone
+    and in the batch.  Members that take the lanes alone and one thread per node in
+    the batch end at the same bits, as do those that take either form in both."""
     if n == 1:
         prm, xc = config.single_sphere(my=my, dia_cells=dia)
     else:
         prm, xc = config.random_array(my=my, dia_cells=dia, nbody=n, seed=n, mc_moves=20)
     prm.update(limiter=limiter, include_frmeanfluid=frfl)
+    alone = _forced_nodes(prm, xc)
+    assert (alone <= FEW_NODES, alone * width <= FEW_NODES) == lanes, alone
     b = pk.Batch([(dict(prm), xc)] * width)
     b.run(3)
     s = pk.Solver(prm, xc)

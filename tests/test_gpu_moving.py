@@ -145,12 +145,15 @@ def test_moving_with_passive_scalar_matches_oracle():
 @pytest.mark.parametrize("my,dia,n,spread,rhos", [(32, 10.0, 1, 0.1, 1e2), (32, 10.0, 5, 3.0, 1e2), (32, 8.0, 31, 0.5, 1e2),
                                                   (64, 12.0, 40, 12.0, 1e2), (64, 8.0, 100, 1.0, 1e2), (64, 6.0, 512, 2.0, 1e2),
                                                   (64, 6.0, 513, 2.0, 1e2), (64, 6.0, 256, 2.0, 1e7), (64, 6.0, 257, 2.0, 1e7),
-                                                  (64, 8.0, 293, 2.0, 1e5)])
+                                                  (64, 8.0, 293, 2.0, 1e5),
+                                                  *((64, 12.0, n, 6.0, 1e2) for n in (9, 14, 18, 22, 27))])
 def test_dem_lists_over_particle_counts(my, dia, n, spread, rhos):
-    """The one-launch DEM (up to 512 spheres, 256 to 512 with few sub-steps
-    to a flow step) and the launches per sub-step: one sphere, fewer than the cluster's warps, more than one per warp,
-    boxes of two and three coarse cells (an image of a sphere through several
-    cells), and spheres fast enough that the candidate lists are rebuilt within a step."""
+    """The one-launch DEM (up to 512 spheres, 256 to 512 with few sub-steps to a
+    flow step) and the launches per sub-step: one sphere, fewer than the
+    cluster's warps, more than one per warp, clusters of every size (a block for
+    four spheres, up to eight), boxes of two and three coarse cells (an image of a
+    sphere through several cells), and spheres fast enough that the candidate
+    lists are rebuilt within a step."""
     rng = np.random.default_rng(n)
     prm, _ = config.single_sphere(my=my, dia_cells=dia, re=20.0)
     prm.update(imove=1, collision_type="softsphere", rhos=rhos, rhof=1.0, coeff_rest=0.9, initialize_zero=True)
