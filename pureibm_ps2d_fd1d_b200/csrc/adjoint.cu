@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(LT * 32) k_adj_lines(Geo g, const double2 *__r
                                                        const double2 *__restrict__ lnl, double2 *__restrict__ lu2,
                                                        double2 *__restrict__ lp2, double2 *__restrict__ lnl_new,
                                                        double2 *__restrict__ lonl, double2 *__restrict__ lff,
-                                                       const Scal *__restrict__ sc, AdjScal *as) {
+                                                       const Scal *__restrict__ sc) {
     constexpr int R = NX / 32;
     constexpr int NP = lines_pitch<NX, LT>();
     extern __shared__ double2 sm[];
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(256) k_adj_q(Geo g, const double2 *__restrict_
     lu2[t] = axpy2(-c12 * g.vis, lap, lu2[t]);
 }
 
-// MUSCL slope of the forward flux (slope_lim) and its partials
+// MUSCL slope of the forward flux (slope_lim_q) and its partials
 // d s / d (u(i-1), u(i), u(i+1)).
 // tdx = 2 dx with its reciprocal rtdx (qdiv).
 __device__ __forceinline__ double slope_d(double um1, double u0, double up1, double tdx, double rtdx, int limiter, double ds[3]) {
@@ -697,7 +697,7 @@ static void enqueue_adjoint_step_t(const Geo &g, const DevBufs &b, const AdjBufs
     const int nsum = 2 * 148;
     k_adj_begin<<<1, 32, 0, s>>>(b.sc, a.as);
     k_adj_lines<N, LT><<<(g.PS + LT - 1) / LT, LT * 32, adj_lines_smem<N>(), s>>>(g, a.lu, a.lp, a.lnl, a.lu2, a.lp2, a.lnl_new,
-                                                                                 a.lonl, a.lff, b.sc, a.as);
+                                                                                 a.lonl, a.lff, b.sc);
     launch_planes<PL<N>>(k_adj_c2r<N>, g.nx, 3, s, g, (const double2 *)a.lff, a.lfr, 0);
     k_adj_sum<N><<<dim3(nsum, 3), 256, 0, s>>>(g, a.lfr, lfrmean, -1.0);
     cudaMemsetAsync(a.lubcp, 0, 10 * CR * sizeof(double), s);   // lubcp, lomega, lpbcp, lpgr

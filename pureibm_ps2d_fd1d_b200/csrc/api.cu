@@ -674,7 +674,8 @@ int pibm_set_state(pibm_handle *h, const pibm_state_view *s) {
     sc.t = s->t; sc.dt = s->dt; sc.cf = s->cf;
     h->next_rks = 1;   // a restart begins a time step
     if (h->g.moving && h->S.dem_soft) {
-        // the step graphs hold max_factor DEM sub-steps; a larger dt needs more
+        // the step graphs hold max_factor: their limit of DEM sub-steps, or their
+        // launches of them; a larger dt needs more
         Mov &m = h->b.mov;
         const int need = std::max(1, (int)(s->dt / m.dtsolid));
         if (need > m.max_factor) {
@@ -719,11 +720,6 @@ int pibm_get_particles(pibm_handle *h, double *pres, double *visc, double *force
 // parity of the nl ping-pong at the slot is kept on the host.
 // ---------------------------------------------------------------------------
 namespace {
-struct SlotSet {
-    char *base = nullptr;
-    size_t bytes = 0;          // per slot
-    std::vector<int> cur;
-};
 size_t slot_bytes(const pibm_handle *h) {
     const size_t SC = (size_t)h->g.nx * h->g.PS * sizeof(double2);
     return 7 * SC + ((sizeof(Scal) + 255) / 256) * 256;
@@ -928,7 +924,7 @@ int pibm_adjoint_run(pibm_handle *h, int nsteps, int checkpoint_every, const dou
     // the work buffers were swapped K times: keep the handle's set consistent
     a = w;
     if (sc_fin.status) return fail(sc_fin.status, "adjoint: a forward step reported a solver stop condition");
-    if (as.status) return fail(as.status, "adjoint: an adjoint kernel reported a bounded-wait timeout or a zero pivot");
+    if (as.status) return fail(as.status, "adjoint: an adjoint kernel reported a bounded-wait timeout");
     for (size_t q = 0; q < gx.size(); ++q) g_xc[q] = gx[q];
     for (int d = 0; d < 3; ++d) g_mpg[d] = as.gmpg[d];
     if (rep) {
@@ -1004,7 +1000,7 @@ int pibm_adjoint_end(pibm_handle *h, double *g_xc, double g_mpg[3]) {
     CUDA_OR_FAIL(cudaMemcpyAsync(gx.data(), h->adj.gxc, gx.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
     if (sc.status) return fail(sc.status, "adjoint: a recomputed step reported a solver stop condition");
-    if (as.status) return fail(as.status, "adjoint: an adjoint kernel reported a bounded-wait timeout or a zero pivot");
+    if (as.status) return fail(as.status, "adjoint: an adjoint kernel reported a bounded-wait timeout");
     if (h->adj_left != 0) return fail(PIBM_ERR_ARG, "pibm_adjoint_end before every step was reversed");
     for (size_t q = 0; q < gx.size(); ++q) g_xc[q] = gx[q];
     for (int d = 0; d < 3; ++d) g_mpg[d] = as.gmpg[d];

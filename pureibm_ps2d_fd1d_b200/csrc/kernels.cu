@@ -216,16 +216,7 @@ __global__ void __launch_bounds__(256) k_scal_a(Geo g, Scal *sc, const double *p
 // k_nl: nonlinear term -div(uu) of one plane (nl_allflow.F90:71-327, nl.F90:99-173).
 // nl_c = -( (wy*F(u_a u_b) + wz*F(u_a' u_b')) + F(D_c) ),  D_c = x-flux difference.
 // ============================================================================
-__device__ __forceinline__ double slope_lim(double um1, double u0, double up1, double dx, int limiter) {
-    double s = (up1 - um1) / (2.0 * dx);
-    double phi = 1.0;
-    if (limiter == PIBM_LIMITER_MINMOD) {
-        phi = (u0 - um1) / (up1 - u0 + kSmallD);
-        phi = phi <= 0.0 ? 0.0 : fmin(1.0, phi);
-    }
-    return s * phi * 1.0;
-}
-// slope_lim with the divisor 2 dx given with its reciprocal (qdiv)
+// MUSCL slope with the limiter; the divisor 2 dx comes with its reciprocal (qdiv)
 __device__ __forceinline__ double slope_lim_q(double um1, double u0, double up1, double tdx, double rtdx, int limiter) {
     double s = qdiv(up1 - um1, tdx, rtdx);
     double phi = 1.0;
@@ -234,51 +225,6 @@ __device__ __forceinline__ double slope_lim_q(double um1, double u0, double up1,
         phi = phi <= 0.0 ? 0.0 : fmin(1.0, phi);
     }
     return s * phi * 1.0;
-}
-
-// x-flux difference D_c at plane i for node e of the plane (upwind: MUSCL
-// states + Rusanov flux, nl_allflow.F90:139-294; center: nl_allflow.F90:97-124,298-310).
-__device__ __forceinline__ double xflux_diff(const Geo &g, const double *__restrict__ ubcp, int i, int e, int c) {
-    const int nx = g.nx;
-    const size_t RS = g.RS;
-    auto U = [&](int comp, int ii) -> double {
-        ii = ii < 0 ? ii + nx : (ii >= nx ? ii - nx : ii);
-        return __ldg(ubcp + ((size_t)comp * nx + ii) * RS + e);
-    };
-    const double dx = g.dx;
-    if (g.scheme == PIBM_SCHEME_CENTER) {
-        const double fp = U(0, i + 1) * U(c, i + 1), fm = U(0, i - 1) * U(c, i - 1);
-        return (fp - fm) / (2.0 * dx);
-    }
-    // cells i-2 .. i+2 of component 0 (advecting velocity) and component c
-    double a[5], b[5];
-#pragma unroll
-    for (int q = 0; q < 5; ++q) { a[q] = U(0, i - 2 + q); b[q] = (c == 0) ? a[q] : U(c, i - 2 + q); }
-    // slopes at cells i-1, i, i+1 (index 1..3 in the window)
-    double sa[3], sb[3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        sa[q] = slope_lim(a[q], a[q + 1], a[q + 2], dx, g.limiter);
-        sb[q] = (c == 0) ? sa[q] : slope_lim(b[q], b[q + 1], b[q + 2], dx, g.limiter);
-    }
-    const double h = dx / 2.0;
-    double F[2];
-#pragma unroll
-    for (int f = 0; f < 2; ++f) {
-        // interface between window cells (f+1) and (f+2): global interface m = i-1+f
-        const double uminus = a[f + 1] + sa[f] * h;
-        const double uplus = a[f + 2] - sa[f + 1] * h;
-        const double Um = b[f + 1] + sb[f] * h;
-        const double Up = b[f + 2] - sb[f + 1] * h;
-        const double Am = 0.5 * uminus * Um, Ap = 0.5 * uplus * Up;
-        const double ms = fmax(fabs(uminus), fabs(uplus));
-        int m = i - 1 + f;
-        m = m < 0 ? m + nx : m;
-        // interface nx (m == nx-1 here, 0-based) receives the cell-1 contribution first
-        const double s = (m == nx - 1) ? ((0.0 + Ap) + Am) : ((0.0 + Am) + Ap);
-        F[f] = s - 0.5 * ms * (Up - Um);
-    }
-    return (F[1] - F[0]) / dx;
 }
 
 // ============================================================================

@@ -196,7 +196,7 @@ __device__ __forceinline__ double2 psrc_term(int n, double c, double2 x0, double
 // Per-line coefficients of velstep's three systems and right-hand sides,
 // every rounding written out (poisson.F90:118-161, usteptime.F90:73-300).
 struct LineCoef {
-    double pa, pb, pc;     // pressure and divcorr systems: a, b, c
+    double pa, pb;         // pressure and divcorr systems: a (= c), b
     double ua, ub;         // ustep system: a (= c), b
     double fy, gd, alp;    // ustep right-hand side: 1 - dt vis c1 w2, dt vis c1, dt (c1 + c2)
     double c2dtv;          // divcorr pressure update: c2 dt vis
@@ -206,7 +206,6 @@ __device__ __forceinline__ LineCoef line_coef(double dt, double vis, double c1, 
     const double r1 = 1.0 / dx2, r2 = -2.0 / dx2, dtv = __dmul_rn(dt, vis);
     k.pa = __dsub_rn(r1, __dmul_rn(0.25, w2));
     k.pb = __dsub_rn(r2, __dmul_rn(0.5, w2));
-    k.pc = k.pa;
     const double dvc2 = __dmul_rn(dtv, c2);
     k.ua = -(dvc2 / dx2);
     k.ub = __dadd_rn(1.0, __dmul_rn(dvc2, __dadd_rn(2.0 / dx2, w2)));

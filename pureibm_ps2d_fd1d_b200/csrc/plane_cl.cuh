@@ -30,13 +30,15 @@
 // The radix twiddles are immediates (cos48); the pass twiddles come from a
 // table of e^{-2 pi i m/N}.
 //
-// Bound: shared-memory wavefronts (4 x 2 plane traversals) and, where one CTA
-// fills its SM, the loads and stores it cannot overlap.  The step's kernels
-// (us per launch at 32 / 64 / 96 / 128 / 256^3; before: five passes, clusters of
-// 2 CTAs at 64-128, radix twiddles from the table):
-//   k_a0  11.2 / 29.2 / 101 / 150 / 1978  ->  10.6 / 21.2 / 56.5 / 141 / 1521
-//   k_nl  14.8 / 40.8 / 119 / 226 / 2036  ->  16.7 / 33.1 / 78.7 / 194 / 2037
-//   k_ff   8.6 / 14.7 / 33.0 / 50.3 / 422 ->   8.5 / 12.6 / 22.6 / 43.8 / 412
+// Bound: no unit is saturated.  At 128^3 k_a0 and k_nl keep the shared-memory pipe
+// (4 x 2 plane traversals) 54 and 48% busy, FP64 and DRAM 22%, and their warps
+// wait for global loads most of all, in k_nl with one CTA to an SM and nothing
+// to run meanwhile.  The step's kernels (us per launch at 32 / 64 / 96 / 128^3;
+// before: five passes, clusters of 2 CTAs at 64-128, radix twiddles from the
+// table; at 256^3 the step transforms by the sweeps of sweep.cuh):
+//   k_a0  11.2 / 29.2 / 101 / 150  ->  10.6 / 21.2 / 56.5 / 141
+//   k_nl  14.8 / 40.8 / 119 / 226  ->  16.7 / 33.1 / 78.7 / 194
+//   k_ff   8.6 / 14.7 / 33.0 / 50.3 ->   8.5 / 12.6 / 22.6 / 43.8
 // (One launch of 1280 planes c2r at 128 with its load and store from HBM: 119 ->
 // 105 us, 53 us at the copy rate; 960 at 96: 78 -> 38 us; 640 at 64: 20.8 -> 12.6 us.)
 #pragma once
@@ -82,10 +84,8 @@ template <int N> using RL = typename PlaneSel<N>::RL;
 template <int N> using NL = typename PlaneSel<N>::NL;
 template <int N> using SL = typename PlaneSel<N>::SL;
 
-// Physical z of shared-memory row R (inverse of zrow), and pair index m of
-// row slot s (inverse of yslot).
+// Physical z of shared-memory row R (inverse of zrow).
 template <int N> __device__ __forceinline__ int zinv(int R) { return (R % Plan<N>::BZ) * Plan<N>::AZ + R / Plan<N>::BZ; }
-template <int N> __device__ __forceinline__ int yinv(int s) { return (s % Plan<N>::BY) * Plan<N>::AY + s / Plan<N>::BY; }
 
 // Global column ky of column-phase slot jl of CTA `rank`.
 template <class L> __device__ __forceinline__ int cl_col(int jl, int rank) { return jl == L::MC ? L::M : rank * L::MC + jl; }

@@ -4,7 +4,7 @@
 //
 // A 256^2 plane needs a cluster of 8 SMs in the plane kernels of plane_cl.cuh,
 // which pay for every element that crosses SMs.  A column or a row is 4 KB:
-// blocks of 32 KB, five or six to an SM, stream them.  The planes in between
+// blocks of 32 KB, four to six to an SM, stream them.  The planes in between
 // cost a write and a read of L2 / HBM; in return
 // the columns' kernels do everything that is local to a (kx-plane, ky) column:
 //   k_cz  inverse z of 7 fields: u(3), p, i kz u1, i kz u2, i kz p, from which
@@ -18,10 +18,10 @@
 // The items (fields, components) of one block of planes run side by side
 // (blockIdx.x), so what they share comes from L2.
 // Measured (us per step at 256^3, plane kernels -> sweeps): fields to real space
-// 1521 -> 1040, nonlinear term 2037 -> 1234, forcing 412 -> 312; the bulk-copied
-// row kernels run at the copy rate (k_rq: 119 us for 810 MB), the column kernels
-// at about 70% of it.  At 128, where a plane fits one SM or two, the two forms
-// are within 2% (141 -> 138, 194 -> 192, 44 -> 48), so it keeps the plane kernels.
+// 1521 -> 958, nonlinear term 2037 -> 1220, forcing 412 -> 311.  At 128, where a
+// plane fits one SM or two, blocks of 8 columns take 132 against 140, 185
+// against 192 and 48 against 44 us, 1% of a step, for 5 launches more: it keeps
+// the plane kernels.
 #pragma once
 #include "step_common.cuh"
 
@@ -29,12 +29,13 @@ namespace pibm {
 
 template <int N> struct Sweep {
     static constexpr int AZ = Plan<N>::AZ, BZ = Plan<N>::BZ, M = N / 2, my2 = M + 1, PS = my2 * N;
-    static constexpr int QC = N >= 256 ? 8 : 16;      // columns of a block: 128 or 256 contiguous bytes per kz
+    static_assert(N == 256, "the only grid that transforms by sweeps (kSweepMin)");
+    static constexpr int QC = 8;                      // columns of a block: 128 contiguous bytes per kz
     static constexpr int NS = M / QC;                 // blocks of a plane (without column M)
     static constexpr int CT = QC * BZ;                // threads of a column block: AZ points of a column each
     static constexpr int GC = N * NS + N / QC;        // blocks of a field: its planes' columns < M, then column M of QC planes each
     static constexpr int CSM = (N * QC + N) * 16;     // shared memory of one column buffer and the twiddles
-    static constexpr int RC = N >= 256 ? 16 : 32;     // rows of a block
+    static constexpr int RC = 16;                     // rows of a block
     static constexpr int RT = 128, RB = N / RC;       // threads, blocks of a plane
     static constexpr int RSM = (RC * my2 + N) * 16;
     static constexpr int RBLK = 6;                    // row blocks per SM the register budget is sized for
