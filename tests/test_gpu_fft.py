@@ -64,7 +64,7 @@ def test_plane_transforms_256_against_numpy():
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,npl", [(32, 1), (32, 149), (64, 3), (96, 1), (96, 297), (128, 149), (256, 2)])
 def test_plane_counts_against_numpy(n, npl):
-    """Every plane shape (one CTA up to 96, clusters above) at plane counts that
+    """Every plane shape (one CTA, clusters of 2 and 8) at plane counts that
     leave SMs idle or a partial last wave; the rounding bound of log2(n^2)
     radix stages is far below the file's tolerance."""
     rng = np.random.default_rng(n + npl)

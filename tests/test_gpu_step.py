@@ -175,10 +175,11 @@ def test_random_array_256_two_steps():
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["fixed", "rk3", "scalar", "moving"])
 def test_repeated_steps_equal_run_across_new_states_and_plans(kind):
-    """Single steps are replayed from recorded launches after the first few:
-    with a state set and the line tiles changed in between they still end at
-    the bits of the same steps as one run, and a state with its scalar field
-    read back and set elsewhere continues alike."""
+    """Single steps are replayed from recorded launches after the first 24 and
+    where run() has recorded them, and launched directly again after a change of
+    the line tiles: with a state set and the tiles changed in between they still
+    end at the bits of the same steps as one run, and a state with its scalar
+    field read back and set elsewhere continues alike."""
     prm, xc = config.random_array(my=32, dia_cells=8, nbody=3, seed=3, mc_moves=50)
     if kind == "rk3":
         prm.update(rk3=True)
@@ -193,9 +194,9 @@ def test_repeated_steps_equal_run_across_new_states_and_plans(kind):
             solver.step(r)
 
     a, b, c = (pk.Solver(P, xc) for _ in range(3))
-    for _ in range(5):
+    for _ in range(27):
         step(a)
-    b.run(5)
+    b.run(27)
     scal = a.get_scalar() if kind == "scalar" else None
     if kind != "moving":   # a moving run's particle state is part of its restart, not of its fields
         st = a.get_state()
@@ -206,14 +207,14 @@ def test_repeated_steps_equal_run_across_new_states_and_plans(kind):
         step(a)
     a.set_tuning(4)
     b.set_tuning(4)
-    for _ in range(4):
+    for _ in range(27):
         step(a)
-    b.run(8)
+    b.run(31)
     solvers = [b]
     if kind != "moving":
         c.run(4)
         c.set_tuning(4)
-        for _ in range(4):
+        for _ in range(27):
             step(c)
         solvers.append(c)
     want = a.get_state()
